@@ -84,6 +84,8 @@ GRETA_API int greta_cuda_memcpy_d2d(void *dst, const void *src, size_t bytes, gr
 /* height rows of width bytes between pitched device arrays, asynchronous on `stream` (hipMemcpy2DAsync in the reference's runtime). */
 GRETA_API int greta_cuda_memcpy_2d_d2d(void *dst, size_t dst_pitch, const void *src, size_t src_pitch, size_t width, size_t height,
                                        greta_stream_t stream);
+/* height rows of width bytes from a pitched device array to a pitched host array; blocks. */
+GRETA_API int greta_cuda_memcpy_2d_d2h_sync(void *dst, size_t dst_pitch, const void *src, size_t src_pitch, size_t width, size_t height);
 GRETA_API int greta_cuda_memcpy_h2d_sync(void *dst, const void *src, size_t bytes);
 GRETA_API int greta_cuda_memcpy_d2h_sync(void *dst, const void *src, size_t bytes);
 GRETA_API int greta_cuda_memset(void *dst, int value, size_t bytes, greta_stream_t stream);

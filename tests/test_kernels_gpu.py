@@ -775,3 +775,22 @@ def test_gemm_rejects_what_it_cannot_do(g):
     assert lib.greta_cuda_gemm(None, g.FMT_F16, buf.ptr, 1, buf.ptr, buf.ptr, buf.ptr, 0, 64, 64, 256, None) == 4     # format
     assert lib.greta_cuda_gemm(None, g.FMT_Q4_0, buf.ptr, 0, buf.ptr, buf.ptr, buf.ptr, 0, 64, 64, 256, None) == 4    # fp32 A without workspace
     assert lib.greta_cuda_gemm(None, g.FMT_Q4_0, None, 1, None, None, None, 0, 0, 64, 256, None) == 0                  # empty
+
+
+@pytest.mark.parametrize("n", [1, 31, 4096, 4097, 8193, 16385, 32003, 128256])
+def test_argmax_over_cta_clusters(g, n):
+    """The first of equal maxima wherever the CTAs of a row's cluster meet; rows of -inf; infinities."""
+    rng = np.random.default_rng(n)
+    rows = rng.normal(0, 1, (3, n)).astype(np.float32)
+    top = np.sort(rng.choice(n, size=min(n, 5), replace=False))
+    rows[0, top] = 9.0
+    rows[1] = -np.inf
+    rows[2, n - 1] = np.inf
+    nxt, pos, cnt = (g.DeviceBuffer(12, zero=True) for _ in range(3))
+    outs = g.DeviceBuffer(3 * 4 * 2, zero=True)
+    lib = g.cuda()
+    for step in range(2):
+        g.check(lib.greta_cuda_argmax_advance_batch(None, _dev(g, rows).ptr, n, 3, nxt.ptr, pos.ptr, outs.ptr, cnt.ptr, 2))
+    assert nxt.download(np.int32).tolist() == [top[0], 0, n - 1]
+    assert outs.download(np.int32).reshape(3, 2).tolist() == [[top[0]] * 2, [0, 0], [n - 1] * 2]
+    assert pos.download(np.int32).tolist() == cnt.download(np.int32).tolist() == [2, 2, 2]
