@@ -214,6 +214,10 @@ int greta_cuda_memcpy_2d_d2d(void *dst, size_t dst_pitch, const void *src, size_
   GRETA_CUDA_TRY(cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, height, cudaMemcpyDeviceToDevice, S(stream)));
   return GRETA_OK;
 }
+int greta_cuda_memcpy_2d_d2h_sync(void *dst, size_t dst_pitch, const void *src, size_t src_pitch, size_t width, size_t height) {
+  GRETA_CUDA_TRY(cudaMemcpy2D(dst, dst_pitch, src, src_pitch, width, height, cudaMemcpyDeviceToHost));
+  return GRETA_OK;
+}
 int greta_cuda_memcpy_h2d_sync(void *dst, const void *src, size_t bytes) {
   GRETA_CUDA_TRY(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
   return GRETA_OK;
