@@ -106,6 +106,35 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ 
   for (uint32_t c = threadIdx.x; c < cols; c += blockDim.x) yr[c] = (xr[c] * inv) * gamma[c];
 }
 
+// The same values as fp16, for the tensor-core products.  A row stays in registers (PER values per thread, all loads under way together;
+// the 256-thread order of the sum is rmsnorm_kernel's, so the results are its bits): 3.8 us for 512 x 4096 in the layer against 10.8 and a
+// conversion pass of 2.9 per product.
+template <int PER>
+__global__ void __launch_bounds__(256) rmsnorm_f16_kernel(const float *x, const float *__restrict__ gamma, __half *y, uint32_t cols, float eps) {
+  __shared__ float sm[32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const float *xr = x + (size_t)blockIdx.x * cols;
+  __half *yr = y + (size_t)blockIdx.x * cols;
+  float v[PER], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const uint32_t c = threadIdx.x + i * 256;
+    v[i] = c < cols ? xr[c] : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) ss = fmaf(v[i], v[i], ss);
+  for (uint32_t c = threadIdx.x + PER * 256; c < cols; c += 256) ss = fmaf(xr[c], xr[c], ss);
+  ss = block_sum(ss, sm);
+  const float inv = rsqrtf(ss / (float)cols + eps);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const uint32_t c = threadIdx.x + i * 256;
+    if (c < cols) yr[c] = __float2half_rn((v[i] * inv) * gamma[c]);
+  }
+  for (uint32_t c = threadIdx.x + PER * 256; c < cols; c += 256) yr[c] = __float2half_rn((xr[c] * inv) * gamma[c]);
+}
+
 __global__ void add_kernel(const float *a, const float *b, float *c, size_t n) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) c[i] = a[i] + b[i];
@@ -302,6 +331,18 @@ int greta_cuda_rmsnorm(greta_stream_t stream, const float *x, const float *gamma
   GRETA_REQUIRE(x && gamma && y, "rmsnorm: null pointer");
   rmsnorm_kernel<<<rows, 256, 0, S(stream)>>>(x, gamma, y, cols, eps);
   return launched("rmsnorm_kernel");
+}
+int greta_cuda_rmsnorm_f16(greta_stream_t stream, const float *x, const float *gamma, void *y, uint32_t rows, uint32_t cols, float eps) {
+  if (rows == 0 || cols == 0) return GRETA_OK;
+  GRETA_REQUIRE(x && gamma && y, "rmsnorm_f16: null pointer");
+  __half *y16 = static_cast<__half *>(y);
+  if (cols <= 256 * 8)
+    GRETA_CUDA_TRY(launch_pdl(rmsnorm_f16_kernel<8>, dim3(rows), dim3(256), 0, S(stream), x, gamma, y16, cols, eps));
+  else if (cols <= 256 * 16)
+    GRETA_CUDA_TRY(launch_pdl(rmsnorm_f16_kernel<16>, dim3(rows), dim3(256), 0, S(stream), x, gamma, y16, cols, eps));
+  else
+    GRETA_CUDA_TRY(launch_pdl(rmsnorm_f16_kernel<32>, dim3(rows), dim3(256), 0, S(stream), x, gamma, y16, cols, eps));
+  return launched("rmsnorm_f16_kernel");
 }
 int greta_cuda_add(greta_stream_t stream, const float *a, const float *b, float *c, size_t n) {
   if (n == 0) return GRETA_OK;

@@ -108,15 +108,6 @@ __device__ __forceinline__ bool rows_paired(const greta_out_segment &g, uint32_t
   return __all_sync(0xffffffffu, same && fits);
 }
 
-// A copy still in flight must not outlive the CTA: after an abort the producer gives the last ones a bounded chance to land.
-__device__ __forceinline__ void drain_copies(uint64_t *full, uint32_t issued, uint32_t stages) {
-  for (uint32_t j = issued > stages ? issued - stages : 0; j < issued; ++j) {
-    const long long t0 = clock64();
-    while (!mbar_try_wait(&full[j % stages], (j / stages) & 1) && clock64() - t0 < 20000000ll) {
-    }
-  }
-}
-
 template <int TN>
 __global__ void __launch_bounds__(DCfg<TN>::THREADS, 1)
 linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ Segments sg, uint32_t M,

@@ -44,6 +44,8 @@ inline int launched(const char *kernel, unsigned n = 1) {
 // predecessor produces (and before it overwrites anything the predecessor reads).  Weight prefetch
 // sits in front of that wait.  pdl_enabled() is read once from GRETA_PDL (default on) and can be
 // switched with greta_cuda_set_pdl().
+// A parameter that the predecessor writes must not be `const T *__restrict__`: such loads count as invariant and the compiler may move them
+// up across the wait (seen: a norm that read rows before the kernel that writes them had ended).
 bool pdl_enabled();
 void set_pdl(bool on);
 

@@ -598,6 +598,31 @@ bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t se
   float *att = static_cast<float *>(a.attn_out.data()), *gate = static_cast<float *>(a.mlp_gate.data()), *up = static_cast<float *>(a.mlp_up.data());
   float *tmp = static_cast<float *>(a.mlp_out.data());
   const bool tp = c.tp_size > 1;
+  // Prompts: products that share their activations in one launch, operands rounded to fp16 where they are made, SwiGLU and residual
+  // in the products' epilogues.  The same roundings as the operator-by-operator form below, which keeps up to 32 rows, other formats and
+  // head sizes.
+  if (S > 32 && (fmt == GRETA_FMT_Q4_0 || fmt == GRETA_FMT_Q8_0) && Dh % 8 == 0 && Dh <= 1024) {
+    void *n16 = a.norm_out.data(), *gate16 = a.mlp_gate.data();  // fp16 rows in buffers sized for fp32
+    const greta_gemm_segment qkv[3] = {{b.wq.data(), b.s_wq.data(), ql, q}, {b.wk.data(), b.s_wk.data(), kvl, k}, {b.wv.data(), b.s_wv.data(), kvl, v}};
+    const greta_gemm_segment ffn[2] = {{b.w1.data(), b.s_w1.data(), hidden_l_, gate16}, {b.w3.data(), b.s_w3.data(), hidden_l_, nullptr}};
+    auto residual = [&](const void *in, Buffer &w, Buffer &sw, uint32_t K, const char *name) -> bool {
+      const greta_gemm_segment g{w.data(), sw.data(), D, tp ? tmp : x};
+      GRETA_TRY(greta_cuda_gemm_segments(s, fmt, in, S, K, &g, 1, tp ? GRETA_GEMM_STORE : GRETA_GEMM_ADD), name);
+      if (!tp) return true;
+      if (all_reduce_(tmp, (size_t)S * D, s) != 0) return fail(err, "all-reduce failed");
+      GRETA_TRY(greta_cuda_add(s, x, tmp, x, (size_t)S * D), "residual");
+      return true;
+    };
+    GRETA_TRY(greta_cuda_rmsnorm_f16(s, x, static_cast<const float *>(b.attn_norm.data()), n16, S, D, c.rms_eps), "rmsnorm");
+    GRETA_TRY(greta_cuda_gemm_segments(s, fmt, n16, S, D, qkv, 3, GRETA_GEMM_STORE), "qkv");
+    GRETA_TRY(greta_cuda_rope_kv(s, q, k, v, kc, vc, S, heads_l_, kv_heads_l_, Dh, c.rope_base, (uint32_t)seq_start, (uint32_t)max_seq_), "rope, kv update");
+    GRETA_TRY(greta_cuda_attn_prefill(s, q, kc, vc, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
+    GRETA_TRY(greta_cuda_f32_to_f16(s, att, q, (size_t)S * ql), "attention output");  // the queries are done with
+    if (!residual(q, b.wo, b.s_wo, ql, "wo")) return false;
+    GRETA_TRY(greta_cuda_rmsnorm_f16(s, x, static_cast<const float *>(b.ffn_norm.data()), n16, S, D, c.rms_eps), "rmsnorm");
+    GRETA_TRY(greta_cuda_gemm_segments(s, fmt, n16, S, D, ffn, 2, GRETA_GEMM_SWIGLU_F16), "w1, w3");
+    return residual(gate16, b.w2, b.s_w2, hidden_l_, "w2");
+  }
   auto proj = [&](const float *in, Buffer &w, Buffer &sw, float *out, uint32_t N, uint32_t K) -> int {
     if (S <= 32) return greta_cuda_gemv(s, fmt, in, 0, w.data(), sw.data(), out, S, N, K);
     return greta_cuda_gemm(s, fmt, in, 0, w.data(), sw.data(), out, 0, S, N, K, a.gemm_ws.data());

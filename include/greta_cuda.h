@@ -313,6 +313,20 @@ GRETA_API int greta_cuda_gemm(greta_stream_t stream, int fmt, const void *A, int
                               const void *qs, const void *d, void *C, int c_is_f16, uint32_t M,
                               uint32_t N, uint32_t K, void *workspace);
 
+/* Up to three products of one prefill operator that share their fp16 activations a_f16 [M x K], one launch: out = half(A) half(dequant(W))^T
+ * with fp32 accumulation, row-major [M x n].  All pointers 16-byte aligned (out: 4); K a multiple of 32.  greta_cuda_gemm_status
+ * reports waits that gave up. */
+#define GRETA_GEMM_STORE 0      /* fp32 results */
+#define GRETA_GEMM_ADD 1        /* added to the fp32 values there */
+#define GRETA_GEMM_SWIGLU_F16 2 /* segments gate and up of one size: fp16 silu(gate) * up to the first segment's out */
+typedef struct greta_gemm_segment {
+  const void *qs, *d;
+  uint32_t n; /* weight rows */
+  void *out;
+} greta_gemm_segment;
+GRETA_API int greta_cuda_gemm_segments(greta_stream_t stream, int fmt, const void *a_f16, uint32_t M, uint32_t K, const greta_gemm_segment *segs,
+                                       uint32_t n_segs, int mode);
+
 /* ------------------------------------------------------------------ attention
  * Decode attention of one query per head over the fp16 KV cache
  * [Hkv][max_seq][Dh], split over the sequence; seq_len = *d_pos + 1 when d_pos
@@ -387,12 +401,18 @@ GRETA_API int greta_cuda_kv_update(greta_stream_t stream, void *k_cache_f16, voi
                                    const float *new_k, const float *new_v, uint32_t S,
                                    uint32_t pos, const uint32_t *d_pos, uint32_t max_seq_len,
                                    uint32_t num_heads_kv, uint32_t head_dim);
+/* greta_cuda_rope on q [S x H x Dh] (in place) and k [S x Hkv x Dh], greta_cuda_kv_update of k and v: one launch.  Dh a multiple of 8 up to 1024,
+ * pointers 16-byte aligned; k is left as it was. */
+GRETA_API int greta_cuda_rope_kv(greta_stream_t stream, float *q, const float *k, const float *v, void *kc, void *vc, uint32_t S, uint32_t H, uint32_t Hkv,
+                                 uint32_t Dh, float base, uint32_t pos, uint32_t max_seq);
 
 /* ------------------------------------------------------------------ small operators */
 /* launch_rmsnorm_naive (basic_kernels.hip:21-64); also what GretaCompute::rmsnorm
  * (greta_compute_hip.cpp:414-419, an empty placeholder in the reference) calls. */
 GRETA_API int greta_cuda_rmsnorm(greta_stream_t stream, const float *x, const float *gamma, float *y,
                                  uint32_t rows, uint32_t cols, float eps);
+/* The same, rounded to fp16. */
+GRETA_API int greta_cuda_rmsnorm_f16(greta_stream_t stream, const float *x, const float *gamma, void *y, uint32_t rows, uint32_t cols, float eps);
 /* launch_add (basic_kernels.hip:127-140). */
 GRETA_API int greta_cuda_add(greta_stream_t stream, const float *a, const float *b, float *c, size_t n);
 /* launch_silu, launch_mul (basic_kernels.hip:141-167), separately. */

@@ -794,3 +794,73 @@ def test_argmax_over_cta_clusters(g, n):
     assert nxt.download(np.int32).tolist() == [top[0], 0, n - 1]
     assert outs.download(np.int32).reshape(3, 2).tolist() == [[top[0]] * 2, [0, 0], [n - 1] * 2]
     assert pos.download(np.int32).tolist() == cnt.download(np.int32).tolist() == [2, 2, 2]
+
+
+class _Segment(C.Structure):
+    _fields_ = [("qs", C.c_void_p), ("d", C.c_void_p), ("n", C.c_uint32), ("out", C.c_void_p)]
+
+
+@pytest.mark.parametrize("name", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("M,K,ns,mode", [(33, 32, (17,), 0), (64, 256, (128,), 0), (257, 1376, (300, 64, 130), 0), (129, 96, (200,), 1), (700, 2048, (384,), 1),
+                                         (2047, 640, (4000, 1000, 1000), 0), (90, 544, (65, 65), 2), (513, 1024, (640, 640), 2)])
+def test_gemm_segments(g, name, M, K, ns, mode):
+    """Up to three products in one launch: one token tile and several per CTA, ragged rows and tokens, K that ends inside a stage and inside a unit of raw
+    weights; stored, added and as SwiGLU.  Stored results are greta_cuda_gemm's bits (same products, same order of K)."""
+    ofmt, gfmt = FMTS[name]
+    rng = np.random.default_rng(M + K)
+    a16 = rng.normal(0, 1, (M, K)).astype(np.float16).view(np.uint16)
+    blk = [make_blocks(rng, ofmt, n, K) for n in ns]
+    w = [g.Weight(b, gfmt, n, K) for b, n in zip(blk, ns)]
+    base = [rng.normal(0, 1, (M + 1, n)).astype(np.float32) for n in ns]
+    outs = [_dev(g, b) for b in base]
+    segs = (_Segment * len(ns))(*[_Segment(x.qs.ptr, x.d.ptr, n, o.ptr) for x, n, o in zip(w, ns, outs)])
+    a = _dev(g, a16)
+    g.check(g.cuda().greta_cuda_gemm_segments(None, gfmt, a.ptr, M, K, C.cast(segs, C.c_void_p), len(ns), mode))
+    g.check(g.cuda().greta_cuda_device_synchronize())
+    assert _gemm_status(g) == 0
+    single = []
+    for x, n in zip(w, ns):
+        c = g.DeviceBuffer(M * n * 4)
+        _KEEP.append(c)
+        g.check(g.cuda().greta_cuda_gemm(None, gfmt, a.ptr, 1, x.qs.ptr, x.d.ptr, c.ptr, 0, M, n, K, None))
+        single.append(c.download(np.float32).reshape(M, n))
+    if mode == 2:
+        z, u = (s.astype(np.float64) for s in single)
+        got = outs[0].download(np.uint16)
+        assert (got[M * ns[0]:] == base[0].view(np.uint16).reshape(-1)[M * ns[0]:]).all()
+        got = O.f16_bits_to_f32(got[:M * ns[0]]).reshape(M, ns[0])
+        want = z / (1 + np.exp(-z)) * u
+        assert (np.abs(got - want) <= 2.0 ** -11 * 1.01 * np.abs(want) + 2.0 ** -24).all()   # one rounding to fp16
+        return
+    for o, b, s in zip(outs, base, single):
+        got = o.download(np.float32).reshape(b.shape)
+        assert (got[M] == b[M]).all()
+        assert (got[:M] == (b[:M] + s if mode == 1 else s)).all()
+
+
+@pytest.mark.parametrize("S,H,Hkv,Dh,pos", [(33, 4, 2, 64, 0), (40, 3, 1, 128, 5), (70, 8, 8, 8, 1)])
+def test_prefill_fused_elementwise(g, S, H, Hkv, Dh, pos):
+    """rope_kv and rmsnorm_f16 give the bits of the operators that they replace."""
+    rng = np.random.default_rng(S)
+    lib, ms = g.cuda(), pos + S + 3
+    q, k, v = (rng.normal(0, 1, (S, h, Dh)).astype(np.float32) for h in (H, Hkv, Hkv))
+    caches = []
+    for fused in (0, 1):
+        dq, dk, dv = _dev(g, q), _dev(g, k), _dev(g, v)
+        kc, vc = (_dev(g, np.zeros((Hkv, ms, Dh), np.uint16)) for _ in range(2))
+        if fused:
+            g.check(lib.greta_cuda_rope_kv(None, dq.ptr, dk.ptr, dv.ptr, kc.ptr, vc.ptr, S, H, Hkv, Dh, 10000.0, pos, ms))
+        else:
+            g.check(lib.greta_cuda_rope(None, dq.ptr, S, H, Dh, 10000.0, pos, None))
+            g.check(lib.greta_cuda_rope(None, dk.ptr, S, Hkv, Dh, 10000.0, pos, None))
+            g.check(lib.greta_cuda_kv_update(None, kc.ptr, vc.ptr, dk.ptr, dv.ptr, S, pos, None, ms, Hkv, Dh))
+        caches.append([dq.download(np.uint32), kc.download(np.uint16), vc.download(np.uint16)])
+    for one, two in zip(*caches):
+        assert (one == two).all()
+    for cols in (7, 2048, 2049, 5000, 9000):
+        x, gm = rng.normal(0, 3, (3, cols)).astype(np.float32), rng.normal(1, 0.1, cols).astype(np.float32)
+        dx, dg, y, h, h2 = _dev(g, x), _dev(g, gm), _dev(g, x), _dev(g, x), _dev(g, x)
+        g.check(lib.greta_cuda_rmsnorm(None, dx.ptr, dg.ptr, y.ptr, 3, cols, 1e-5))
+        g.check(lib.greta_cuda_f32_to_f16(None, y.ptr, h.ptr, 3 * cols))
+        g.check(lib.greta_cuda_rmsnorm_f16(None, dx.ptr, dg.ptr, h2.ptr, 3, cols, 1e-5))
+        assert (h.download(np.uint16)[:3 * cols] == h2.download(np.uint16)[:3 * cols]).all()
