@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
   const uint32_t tmem = *tmem_slot, tmem_w = tmem + TS_TMEM - TS * TS_W_COLS;
   pdl_launch_dependents();
 
+  const bool leader = elect_one();
   if (warp == 0) {
     pdl_wait();
     uint32_t s = 0, ph = 1, issued = 0;
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
       for (uint32_t kt = 0; kt < KT; ++kt) {
         ok = mbar_wait(&act_empty[s], ph, abort_flag, 100 + s);
         if (!ok) break;
-        if (elect_one()) {
+        if (leader) {
           uint8_t *dst = act + (size_t)s * act_bytes;
           mbar_arrive_expect_tx(&act_full[s], act_bytes);
           tma_load_2d(dst, &w.act, (int)(kt * TS_K), m0, &act_full[s]);
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
         if (u == TS_RAW_UNITS) pdl_wait();  // from here on the bounded waits depend on the predecessor's end
         ok = mbar_wait(&raw_empty[slot], ((u / TS_RAW_UNITS) & 1) ^ 1, abort_flag, 200 + slot);
         if (!ok) break;
-        if (elect_one()) {
+        if (leader) {
           uint8_t *dst = raw + slot * TS_RAW_BYTES;
           const int kd = (int)((Q4 ? kq : kq / 2) * 8);  // the scales of 256 elements
           mbar_arrive_expect_tx(&raw_full[slot], TS_RAW_BYTES);
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
         if (!ok) break;
         ++g;
         tc_fence_after();
-        if (elect_one()) {
+        if (leader) {
           const uint32_t d = tmem + b * TN, a = tmem_w + slot * TS_W_COLS;
 #pragma unroll
           for (uint32_t k16 = 0; k16 < TS_K / 16; ++k16)
@@ -183,14 +184,12 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
           umma_commit(&w_empty[slot]);
           umma_commit(&act_empty[s]);
         }
-        __syncwarp();
         if (++s == AS) {
           s = 0;
           ph ^= 1;
         }
       }
-      if (ok && elect_one()) umma_commit(&acc_full[b]);
-      __syncwarp();
+      if (ok && leader) umma_commit(&acc_full[b]);
     }
   } else if (warp >= (int)TS_DEQ_WARP0 && warp < (int)TS_EPI_WARP0) {
     // The set of a stage is its weight slot, and with whole units in every tile a raw slot is always read by the same sets: whoever waits on
@@ -210,7 +209,6 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
             after = true;
           }
           ok = mbar_wait(&raw_full[slot], (u / TS_RAW_UNITS) & 1, abort_flag, 400 + slot);
-          if (!ok) break;
           const uint8_t *st = raw + slot * TS_RAW_BYTES, *pr = st + row * 128;
           const uint2 dw = *reinterpret_cast<const uint2 *>(st + TS_RAW_PAYLOAD + row * 16 + (Q4 ? sub : kq & 1) * 8);
           uint32_t v[32];  // 64 fp16 of the row, ascending K; past K the copies filled payload, scales and activations with zeros
@@ -253,10 +251,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
               }
             }
             if (half == 0) {
-              ok = mbar_wait(&w_empty[set], ((g >> lg) & 1) ^ 1, abort_flag, 410 + set);
+              ok = __all_sync(0xffffffffu, ok && mbar_wait(&w_empty[set], ((g >> lg) & 1) ^ 1, abort_flag, 410 + set));  // both waits, by the whole warp
               if (!ok) break;
               tc_fence_after();
-              __syncwarp();
             }
             tmem_st32(tmem_w + set * TS_W_COLS + half * 32 + ((quad * 32) << 16), v);
           }
@@ -279,7 +276,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
       const uint32_t N = w.n[seg], row = (rt - (seg ? w.tile_end[seg - 1] : 0)) * TILE_ROWS + in_tile, cols = min(TN, w.M - m0);
       const uint32_t src = tmem + b * TN + ((quad * 32) << 16), par = (w.accs == 2 ? it >> 1 : it) & 1;
       if (PAIR) {
-        if (!all_of_128(mbar_wait(&acc_full[b], par, abort_flag, 500 + b))) break;  // all four warps leave together: they meet at barriers below
+        if (!all_of_128(mbar_wait_warp(&acc_full[b], par, abort_flag, 500 + b))) break;  // all four warps leave together: they meet at barriers below
         tc_fence_after();
         // Of 32 columns the gate warps hand over the last 16 and finish the first 16, the up warps the other way round.
         const bool up = quad >= 2;
@@ -311,7 +308,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
           for (uint32_t j = 0; j < 16; ++j) old[j] = row < N && c + j < cols ? o[(size_t)(c + j) * N] : 0.f;
         };
         if (MODE == GRETA_GEMM_ADD) fetch(0);  // the residual of the next 16 columns is on its way while these are stored
-        if (!mbar_wait(&acc_full[b], par, abort_flag, 500 + b)) break;
+        if (!mbar_wait_warp(&acc_full[b], par, abort_flag, 500 + b)) break;
         tc_fence_after();
 #pragma unroll 1
         for (uint32_t c = 0; c < cols; c += MODE == GRETA_GEMM_ADD ? 16 : 32) {

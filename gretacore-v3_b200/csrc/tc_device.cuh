@@ -84,13 +84,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow<true>(smem_u32(bar), parity, abort_flag, code);
 }
+// The same by a whole warp that goes on together (tcgen05.ld / st, __syncwarp): all lanes succeed or all give up.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code));
+}
 // The same for waits on a kernel's critical path: polls without sleeping.
 __device__ __forceinline__ bool mbar_wait_now(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int code) {
   return mbar_wait_slow<false>(smem_u32(bar), parity, abort_flag, code);
 }
-// One lane of a converged warp, the same one every time.  A warp that issues MMAs, commits or TMA copies runs its loop with all lanes and
-// issues under this predicate: values stay warp-uniform for the compiler, where `if (lane == 0) { loop }` made every tcgen05 and barrier
-// instruction convert its operands (86 instead of 64 us for 172 stages of 64 K x 128 tokens).
+// One lane of a converged warp.  A warp that issues MMAs, commits or TMA copies runs its loop with all lanes and issues where this is true:
+// loop counters and addresses stay warp-uniform for the compiler, where `if (lane == 0) { loop }` made every tcgen05 and barrier
+// instruction convert its operands (86 instead of 64 us for 172 stages of 64 K x 128 tokens).  Asked once, in front of the loop: a lane whose
+// bounded wait gives up may leave the loop alone, so nothing inside may need the whole warp.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
