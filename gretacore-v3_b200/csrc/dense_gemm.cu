@@ -120,7 +120,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   uint64_t *full = bars, *empty = bars + ST, *acc_full = bars + 2 * ST, *acc_empty = acc_full + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t KT = (K + BK - 1) / BK, tok_tiles = (M + TN - 1) / TN, tiles = tok_tiles * ((N + TILE_N - 1) / TILE_N);
 
   if (threadIdx.x == 0) {
@@ -148,54 +148,55 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   pdl_launch_dependents();
   pdl_wait();
 
+  const bool leader = elect_one();
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t issued = 0, s = 0, ph = 1;
-      bool ok = true;
-      for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const int n0 = (int)(t / tok_tiles) * TILE_N, m0 = (int)(t % tok_tiles) * TN;
-        for (uint32_t kt = 0; kt < KT; ++kt) {
-          ok = mbar_wait(&empty[s], ph, abort_flag, 100 + s);
-          if (!ok) break;
-          uint8_t *st = smem + (size_t)s * C::STAGE;
+    uint32_t issued = 0, s = 0, ph = 1;
+    bool ok = true;
+    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+      const int n0 = (int)(t / tok_tiles) * TILE_N, m0 = (int)(t % tok_tiles) * TN;
+      for (uint32_t kt = 0; kt < KT; ++kt) {
+        ok = mbar_wait(&empty[s], ph, abort_flag, 100 + s);
+        if (!ok) break;
+        uint8_t *st = smem + (size_t)s * C::STAGE;
+        if (leader) {
           mbar_arrive_expect_tx(&full[s], C::STAGE);
           tma_load_2d(st, &tmap_w, (int)(kt * BK), n0, &full[s]);
           tma_load_2d(st + C::A_BYTES, &tmap_x, (int)(kt * BK), m0, &full[s]);
-          ++issued;
-          if (++s == ST) {
-            s = 0;
-            ph ^= 1;
-          }
+        }
+        ++issued;
+        if (++s == ST) {
+          s = 0;
+          ph ^= 1;
         }
       }
-      if (*abort_flag) drain_copies(full, issued, ST);
     }
+    if (*abort_flag) drain_copies(full, issued, ST);
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t lo0 = smem_desc_lo(smem_u32(smem));
-      uint32_t s = 0, ph = 0, it = 0;
-      bool ok = true;
-      for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
-        const uint32_t b = it & 1;
-        ok = mbar_wait(&acc_empty[b], ((it >> 1) & 1) ^ 1, abort_flag, 300 + b);
+    const uint32_t lo0 = smem_desc_lo(smem_u32(smem));
+    uint32_t s = 0, ph = 0, it = 0;
+    bool ok = true;
+    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+      const uint32_t b = it & 1;
+      ok = mbar_wait(&acc_empty[b], ((it >> 1) & 1) ^ 1, abort_flag, 300 + b);
+      if (!ok) break;
+      tc_fence_after();
+      for (uint32_t kt = 0; kt < KT; ++kt) {
+        ok = mbar_wait(&full[s], ph, abort_flag, 200 + s);
         if (!ok) break;
         tc_fence_after();
-        for (uint32_t kt = 0; kt < KT; ++kt) {
-          ok = mbar_wait(&full[s], ph, abort_flag, 200 + s);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t w_lo = lo0 + s * (C::STAGE >> 4), x_lo = w_lo + (C::A_BYTES >> 4);
+        const uint32_t w_lo = lo0 + s * (C::STAGE >> 4), x_lo = w_lo + (C::A_BYTES >> 4);
+        if (leader) {
 #pragma unroll
           for (int k16 = 0; k16 < BK / 16; ++k16)
             umma_f16(tmem_base + b * TN, w_lo + k16 * 2, x_lo + k16 * 2, SMEM_DESC_HI_SW128, idesc, (kt | k16) ? 1u : 0u);
           umma_commit(&empty[s]);
-          if (++s == ST) {
-            s = 0;
-            ph ^= 1;
-          }
         }
-        if (ok) umma_commit(&acc_full[b]);
+        if (++s == ST) {
+          s = 0;
+          ph ^= 1;
+        }
       }
+      if (ok && leader) umma_commit(&acc_full[b]);
     }
   } else {
     constexpr int SHARE = TN / (C::EPI_WARPS / 4);  // tokens per warp
@@ -214,7 +215,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         if (g.bias) bias = __ldg(g.bias + r);
       }
       const bool paired = rows_paired(g, r, which, row < N);
-      if (!mbar_wait(&acc_full[b], (it >> 1) & 1, abort_flag, 400 + b)) break;
+      if (!mbar_wait_warp(&acc_full[b], (it >> 1) & 1, abort_flag, 400 + b)) break;
       tc_fence_after();
 #pragma unroll 1
       for (int c = c_begin; c < c_begin + SHARE; c += 32) {
@@ -260,7 +261,7 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   float *part = reinterpret_cast<float *>(smem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t KT = (K + BK - 1) / BK, tok_tiles = (M + TN - 1) / TN, tile = blockIdx.x / S;
   const uint32_t n0 = (tile / tok_tiles) * TILE_N, m0 = (tile % tok_tiles) * TN;
   const uint32_t kt0 = KT * rank / S, kt1 = KT * (rank + 1) / S;  // the plan leaves every CTA some stages
@@ -287,48 +288,49 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   pdl_launch_dependents();
   pdl_wait();
 
+  const bool leader = elect_one();
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t issued = 0, s = 0, ph = 1;
-      for (uint32_t kt = kt0; kt < kt1; ++kt) {
-        if (!mbar_wait(&empty[s], ph, abort_flag, 100 + s)) break;
-        uint8_t *st = smem + (size_t)s * C::STAGE;
+    uint32_t issued = 0, s = 0, ph = 1;
+    for (uint32_t kt = kt0; kt < kt1; ++kt) {
+      if (!mbar_wait(&empty[s], ph, abort_flag, 100 + s)) break;
+      uint8_t *st = smem + (size_t)s * C::STAGE;
+      if (leader) {
         mbar_arrive_expect_tx(&full[s], C::STAGE);
         tma_load_2d(st, &tmap_w, (int)(kt * BK), (int)n0, &full[s]);
         tma_load_2d(st + C::A_BYTES, &tmap_x, (int)(kt * BK), (int)m0, &full[s]);
-        ++issued;
-        if (++s == ST) {
-          s = 0;
-          ph ^= 1;
-        }
       }
-      if (*abort_flag) drain_copies(full, issued, ST);
+      ++issued;
+      if (++s == ST) {
+        s = 0;
+        ph ^= 1;
+      }
     }
+    if (*abort_flag) drain_copies(full, issued, ST);
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t lo0 = smem_desc_lo(smem_u32(smem));
-      uint32_t s = 0, ph = 0;
-      bool ok = true;
-      for (uint32_t kt = kt0; kt < kt1; ++kt) {
-        ok = mbar_wait(&full[s], ph, abort_flag, 200 + s);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t w_lo = lo0 + s * (C::STAGE >> 4), x_lo = w_lo + (C::A_BYTES >> 4);
+    const uint32_t lo0 = smem_desc_lo(smem_u32(smem));
+    uint32_t s = 0, ph = 0;
+    bool ok = true;
+    for (uint32_t kt = kt0; kt < kt1; ++kt) {
+      ok = mbar_wait(&full[s], ph, abort_flag, 200 + s);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t w_lo = lo0 + s * (C::STAGE >> 4), x_lo = w_lo + (C::A_BYTES >> 4);
+      if (leader) {
 #pragma unroll
         for (int k16 = 0; k16 < BK / 16; ++k16)
           umma_f16(tmem_base, w_lo + k16 * 2, x_lo + k16 * 2, SMEM_DESC_HI_SW128, idesc, (kt > kt0 || k16) ? 1u : 0u);
         umma_commit(&empty[s]);
-        if (++s == ST) {
-          s = 0;
-          ph ^= 1;
-        }
       }
-      if (ok) umma_commit(acc_full);
+      if (++s == ST) {
+        s = 0;
+        ph ^= 1;
+      }
     }
+    if (ok && leader) umma_commit(acc_full);
   } else {
     constexpr int SHARE = TN / (C::EPI_WARPS / 4);
     const int quad = warp & 3, c_begin = ((warp - 2) >> 2) * SHARE;
-    if (mbar_wait(acc_full, 0, abort_flag, 400)) {  // every stage has been loaded and multiplied: the ring is idle
+    if (mbar_wait_warp(acc_full, 0, abort_flag, 400)) {  // every stage has been loaded and multiplied: the ring is idle
       tc_fence_after();
 #pragma unroll 1
       for (int c = c_begin; c < c_begin + SHARE; c += 32) {
