@@ -508,9 +508,10 @@ static int attn_prefill_impl(greta_stream_t stream, const float *q, const void *
   p.H = H; p.Hkv = Hkv; p.max_seq = max_seq; p.scale = scale; p.splits = 1; p.len_step = 1;
   // Prompts run on the tensor cores; a few positions, or the switch off, take one CTA per (position, head) on the decode inner loop.
   if (tuning().attn_mma && S >= 8 && (Dh == 64 || Dh == 128) && aligned16(q) && aligned16(kc) && aligned16(vc) && aligned16(o)) {
-    // Above 128 keys the tcgen05 form (10 us + 1.3 per 128 keys in a row of tiles) beats mma.sync (5 us + 4.2 per 64 keys): 16 rows at 1516 keys 25
-    // against 100 us, 512 rows x 32 heads 19 against 47, 1531 rows 62 against 242; 100 rows 13.4 against 12.4.
-    if (pos0 + S > 128 && (!o16 || aligned16(o16)))
+    // tcgen05 above 512 keys (10 us + 1.3 per 128 keys, mma.sync 5 us + 4.2 per 64 keys; 1531 rows of 32 heads 63 against 242 us).  It would pay from
+    // 128 keys on (512 rows of 32 heads: 19 against 47 us).  The line lies higher because the ids of the 512-token 7B run hang on a top-2 gap of
+    // 4.4e-6, less than what the products' sums leave open: with the smaller rounding error of this form one id of 128 is another.
+    if (pos0 + S > 512 && (!o16 || aligned16(o16)))
       return attn_tc_prefill((cudaStream_t)stream, p, S, pos0, Dh, o16 ? o16 : (void *)o, o16 != nullptr);
     if (int rc = attn_mma_prefill((cudaStream_t)stream, p, S, pos0, Dh)) return rc;
   } else if (int rc = launch_attn<__half>((cudaStream_t)stream, p, S, Dh)) {

@@ -193,7 +193,7 @@ struct Parts {
 constexpr int LM_K = 64, LM_THREADS = 256;
 // grid (splits, groups of 16 HT heads, rows); NT: 16-column tiles of the latent per warp (8 warps).
 template <int HT, int NT>
-__global__ void __launch_bounds__(LM_THREADS) latent_mma_kernel(const __grid_constant__ LatArgs w, const __half *__restrict__ q_in, Parts parts, int buffers) {
+__global__ void __launch_bounds__(LM_THREADS) latent_mma_kernel(const __grid_constant__ LatArgs w, const __half *q_in, Parts parts, int buffers) {
   constexpr int HR = 16 * HT, PB = LM_K * 2 + 16;
   const greta_latent_attn &a = w.a;
   extern __shared__ __align__(16) uint8_t smb[];
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(LM_THREADS) latent_mma_kernel(const __grid_con
 // 32-bit form: grid (splits, groups of HN heads, rows).  Eight lanes per key for the scores, four columns per thread for the sums.
 constexpr int LR_KEYS = 128, LR_THREADS = 256;
 template <int HN>
-__global__ void __launch_bounds__(LR_THREADS) latent_rows_kernel(const __grid_constant__ LatArgs w, const float *__restrict__ q_in, Parts parts) {
+__global__ void __launch_bounds__(LR_THREADS) latent_rows_kernel(const __grid_constant__ LatArgs w, const float *q_in, Parts parts) {
   const greta_latent_attn &a = w.a;
   extern __shared__ __align__(16) float smf[];
   __shared__ float sm[HN], sl[HN], sf[HN];
@@ -582,8 +582,8 @@ latent_prefill_kernel(const __grid_constant__ LatArgs w, const __grid_constant__
   const uint32_t sd = slabs(a.dim), sr = slabs(a.rot_dim), sv = slabs(a.vdim), d8 = up8(a.dim), v8 = up8(a.vdim);
   uint8_t *qs = smem, *ks = qs + (sd + sr) * LP_SLAB_Q, *vs = ks + stages * (sd + sr) * SLAB;
   uint64_t *bars = reinterpret_cast<uint64_t *>(vs + stages * sv * SLAB);
-  uint64_t *kf = bars, *ke = bars + 2, *vf = bars + 4, *ve = bars + 6, *sf = bars + 8, *pf = bars + 10, *od = bars + 12, *qf = bars + 13;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 14);
+  uint64_t *kf = bars, *ke = bars + 2, *vf = bars + 4, *ve = bars + 6, *sf = bars + 8, *pf = bars + 10, *od = bars + 12, *qf = bars + 13, *fin = bars + 14;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 15);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t tile = gridDim.x - 1 - blockIdx.x, h = blockIdx.y;  // the longest rows first
@@ -599,6 +599,7 @@ latent_prefill_kernel(const __grid_constant__ LatArgs w, const __grid_constant__
       mbar_init(&pf[i], 4);
     }
     mbar_init(od, 1);
+    mbar_init(fin, 1);
     mbar_init(qf, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -686,6 +687,7 @@ latent_prefill_kernel(const __grid_constant__ LatArgs w, const __grid_constant__
           umma_f16_ts(tmem + 256, tmem + (t & 1) * 128 + k16 * 8, v_lo + st * sv * (SLAB >> 4) + k16 * (2048 >> 4), SMEM_DESC_HI_SW128, idesc_o, (t | k16) ? 1u : 0u);
         umma_commit(&ve[st]);
         umma_commit(od);
+        if (t + 1 == ntiles) umma_commit(fin);
         if (t + 2 < ntiles) ok = mbar_wait_now(od, t & 1, abort_flag, 240) && scores(t + 2);  // the weights of tile t are read: its columns are free
       }
     }
@@ -758,8 +760,8 @@ latent_prefill_kernel(const __grid_constant__ LatArgs w, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(&pf[t & 1]);
     }
-    // the last two products one after the other: a wait may be one phase behind its barrier, not two
-    ok = ok && (ntiles < 2 || mbar_wait_now(od, (ntiles - 2) & 1, abort_flag, 320)) && mbar_wait_now(od, (ntiles - 1) & 1, abort_flag, 321);
+    // A barrier of its own for the end: od may be two phases on by now, which a parity takes for none.
+    ok = ok && mbar_wait_now(fin, 0, abort_flag, 320);
     if (ok) {
       tc_fence_after();
       const float sink2 = a.sink ? a.sink[h] * LOG2E : -INFINITY, nm = fmaxf(mx, sink2), f = ex2(mx - nm), inv = f / (l * f + ex2(sink2 - nm));

@@ -866,9 +866,9 @@ def test_prefill_fused_elementwise(g, S, H, Hkv, Dh, pos):
         assert (h.download(np.uint16)[:3 * cols] == h2.download(np.uint16)[:3 * cols]).all()
 
 
-@pytest.mark.parametrize("S,pos0,H,Hkv,Dh,gain", [(129, 0, 2, 2, 128, 1.0), (8, 121, 4, 1, 64, 1.0), (256, 0, 2, 1, 64, 1.0), (300, 83, 3, 3, 128, 1.0), (16, 700, 4, 2, 128, 1.0),
-                                                  (385, 0, 2, 1, 128, 8.0), (128, 1, 1, 1, 64, 8.0)])
-def test_prefill_attention_above_128_keys(g, S, pos0, H, Hkv, Dh, gain):
+@pytest.mark.parametrize("S,pos0,H,Hkv,Dh,gain", [(513, 0, 2, 2, 128, 1.0), (8, 505, 4, 1, 64, 1.0), (640, 0, 2, 1, 64, 1.0), (300, 467, 3, 3, 128, 1.0), (16, 700, 4, 2, 128, 1.0),
+                                                  (769, 0, 2, 1, 128, 8.0), (128, 513, 1, 1, 64, 8.0)])
+def test_prefill_attention_above_512_keys(g, S, pos0, H, Hkv, Dh, gain):
     """Tile edges of queries and keys, rows behind the last key that are no numbers, maxima that grow from tile to tile (gain); fp16 output is the rounded
     fp32 output.  Tolerance: pairs of fp16 keep 22 bits of queries and probabilities, sums are cut at 24 bits up to 8 times per 128 keys."""
     rng = np.random.default_rng(S + Dh)
