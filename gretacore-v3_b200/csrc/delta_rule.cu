@@ -452,7 +452,7 @@ struct OutArgs {
   float eps;
 };
 template <int LPH, bool VEC>
-__global__ void __launch_bounds__(256) delta_output_kernel(const __grid_constant__ OutArgs d, const float *__restrict__ o_buf, void *out, int out_fmt,
+__global__ void __launch_bounds__(256) delta_output_kernel(const __grid_constant__ OutArgs d, const float *o_buf, void *out, int out_fmt,
                                                            uint32_t ld_out) {
   constexpr int PER = VEC ? 4 : 1, MAXU = VEC ? 2 : 8;  // units per lane: LPH * MAXU * PER >= 256 channels for the widest heads
   pdl_launch_dependents();

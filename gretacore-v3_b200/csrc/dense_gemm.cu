@@ -381,7 +381,7 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
 }
 
 // C tile 64 rows of x x 64 rows of W, 256 threads, 4 x 4 outputs each, 16 columns per step.
-__global__ void __launch_bounds__(256) linear_f32_kernel(const float *__restrict__ W, uint32_t N, uint32_t ldw, const float *__restrict__ x, uint32_t ldx,
+__global__ void __launch_bounds__(256) linear_f32_kernel(const float *__restrict__ W, uint32_t N, uint32_t ldw, const float *x, uint32_t ldx,
                                                          uint32_t M, const __grid_constant__ Segments sg) {
   __shared__ float ws[16][68], xs[16][68];
   pdl_launch_dependents();

@@ -507,7 +507,7 @@ constexpr int PREP_THREADS = 512;
 constexpr size_t PREP_HEADER = 256;
 
 template <int FMT, int MT>
-__global__ void __launch_bounds__(PREP_THREADS) prep_rows_kernel(const float *__restrict__ x, const float *__restrict__ gamma, float eps, uint32_t M,
+__global__ void __launch_bounds__(PREP_THREADS) prep_rows_kernel(const float *x, const float *__restrict__ gamma, float eps, uint32_t M,
                                                                  uint32_t K, uint8_t *__restrict__ ws) {
   __shared__ float red_max[PREP_THREADS / 32], red_ss[PREP_THREADS / 32];
   pdl_launch_dependents();

@@ -253,7 +253,7 @@ constexpr int WR_KEYS = 256, WR_THREADS = 256, KPG = 4;  // keys of a pass; keys
 
 // grid (splits, kv heads * head passes, rows), cluster (splits, 1, 1); HN query heads of one key/value head per CTA.
 template <typename CT, int HN, bool FUSED>
-__global__ void __launch_bounds__(WR_THREADS) window_rows_kernel(const __grid_constant__ WinArgs w, const float *__restrict__ q_in, void *out, int out_fmt,
+__global__ void __launch_bounds__(WR_THREADS) window_rows_kernel(const __grid_constant__ WinArgs w, const float *q_in, void *out, int out_fmt,
                                                                  uint32_t ld_out) {
   const greta_window_attn &a = w.a;
   extern __shared__ __align__(16) float smem[];
@@ -469,7 +469,7 @@ struct MmaCfg {
 
 // grid (query tiles, heads); DB: head size bucket (64, 128 or 256) for both dim and vdim, unused columns zero.
 template <int DB>
-__global__ void __launch_bounds__(WM_THREADS) window_mma_kernel(const __grid_constant__ WinArgs w, const float *__restrict__ q_in, void *out, int out_fmt,
+__global__ void __launch_bounds__(WM_THREADS) window_mma_kernel(const __grid_constant__ WinArgs w, const float *q_in, void *out, int out_fmt,
                                                                 uint32_t ld_out) {
   constexpr int ROWP = MmaCfg<DB>::ROWP;
   constexpr float LOG2E = 1.4426950408889634f;
