@@ -35,7 +35,6 @@ using namespace greta;
 
 namespace greta {
 int gemm_ts_status(int *code);  // gemm_ts.cu
-int attn_tc_status(int *code);  // attention_tc.cu
 }
 
 namespace {
@@ -1125,9 +1124,7 @@ int greta_cuda_gemm_route(uint32_t M, uint32_t N, uint32_t K, int has_workspace,
 int greta_cuda_gemm_status(int *code) {
   GRETA_REQUIRE(code, "gemm_status: null out pointer");
   GRETA_CUDA_TRY(cudaMemcpyFromSymbol(code, g_gemm_error, sizeof(int)));
-  if (*code) return GRETA_OK;
-  if (int rc = gemm_ts_status(code)) return rc;
-  return *code ? GRETA_OK : attn_tc_status(code);
+  return *code ? GRETA_OK : gemm_ts_status(code);
 }
 
 int greta_cuda_gemm(greta_stream_t stream, int fmt, const void *A, int a_is_f16, const void *qs, const void *d, void *Cout, int c_is_f16,

@@ -616,15 +616,9 @@ bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t se
     GRETA_TRY(greta_cuda_rmsnorm_f16(s, x, static_cast<const float *>(b.attn_norm.data()), n16, S, D, c.rms_eps), "rmsnorm");
     GRETA_TRY(greta_cuda_gemm_segments(s, fmt, n16, S, D, qkv, 3, GRETA_GEMM_STORE), "qkv");
     GRETA_TRY(greta_cuda_rope_kv(s, q, k, v, kc, vc, S, heads_l_, kv_heads_l_, Dh, c.rope_base, (uint32_t)seq_start, (uint32_t)max_seq_), "rope, kv update");
-    void *att16 = n16;  // its rows of 2 D halves are free by now
-    if (ql <= 2 * D) {
-      GRETA_TRY(greta_cuda_attn_prefill_f16(s, q, kc, vc, att16, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
-    } else {
-      att16 = q;
-      GRETA_TRY(greta_cuda_attn_prefill(s, q, kc, vc, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
-      GRETA_TRY(greta_cuda_f32_to_f16(s, att, att16, (size_t)S * ql), "attention output");  // the queries are done with
-    }
-    if (!residual(att16, b.wo, b.s_wo, ql, "wo")) return false;
+    GRETA_TRY(greta_cuda_attn_prefill(s, q, kc, vc, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
+    GRETA_TRY(greta_cuda_f32_to_f16(s, att, q, (size_t)S * ql), "attention output");  // the queries are done with
+    if (!residual(q, b.wo, b.s_wo, ql, "wo")) return false;
     GRETA_TRY(greta_cuda_rmsnorm_f16(s, x, static_cast<const float *>(b.ffn_norm.data()), n16, S, D, c.rms_eps), "rmsnorm");
     GRETA_TRY(greta_cuda_gemm_segments(s, fmt, n16, S, D, ffn, 2, GRETA_GEMM_SWIGLU_F16), "w1, w3");
     return residual(gate16, b.w2, b.s_w2, hidden_l_, "w2");
