@@ -217,10 +217,6 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
             uint4 q[Q4 ? 2 : 4];
 #pragma unroll
             for (int c = 0; c < (Q4 ? 2 : 4); ++c) q[c] = *reinterpret_cast<const uint4 *>(pr + (((Q4 ? sub * 4 + half * 2 + c : half * 4 + c) ^ x7) << 4));
-            if (half == 1) {
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&raw_empty[slot]);
-            }
 #pragma unroll
             for (int hb = 0; hb < 2; ++hb) {
               const uint32_t w2 = half ? dw.y : dw.x, dh = hb ? (w2 >> 16) : (w2 & 0xFFFFu), d2 = dh | (dh << 16);
@@ -261,7 +257,13 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&w_full[set]);
+          // The raw unit is given back here, where every loaded value has been used, and not behind its last load: a load under way is not ahead
+          // of the arrival, nor of the copy that the arrival lets loose (seen: single weight rows of a SwiGLU tile multiplied with the unit
+          // that followed, in most prompts of more than 1000 tokens).
+          if (lane == 0) {
+            mbar_arrive(&w_full[set]);
+            mbar_arrive(&raw_empty[slot]);
+          }
         }
       }
     }

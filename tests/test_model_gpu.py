@@ -93,6 +93,29 @@ def test_long_prompt_takes_the_tensor_core_route_and_matches_oracle(pkg):
     m.close()
 
 
+@pytest.mark.parametrize("tokens,fmt_name", [(257, "q4_0"), (1531, "q8_0"), (3001, "q4_0")])
+def test_whole_prompts_give_the_same_bits_every_time(pkg, tokens, fmt_name):
+    """One prompt on one model and on a fresh one, kernels started ahead of their predecessor's end and not (greta_cuda_set_pdl): hidden rows and logits
+    are the same bits.  The feed-forward products of the longer prompts are up to 25 tiles per CTA, so every ring in them is reused many times."""
+    cfg = dict(dim=2048, num_heads=16, num_heads_kv=4, num_layers=2, vocab=1000, hidden_dim=14336, head_dim=128, max_seq=tokens, rope_base=500000.0, rms_eps=1e-5)
+    gfmt = pkg.ffi.FMT_Q4_0 if fmt_name == "q4_0" else pkg.ffi.FMT_Q8_0
+    prompt = pkg.model.synth_tokens(17, tokens, cfg["vocab"])
+    lib, first = pkg.ffi.cuda(), None
+    try:
+        for _ in range(2):
+            m = pkg.model.Model(cfg, weight_fmt=gfmt)
+            m.load_synthetic(17)
+            for pdl in (0, 1, 1, 1):
+                pkg.ffi.check(lib.greta_cuda_set_pdl(pdl))
+                got = [m.forward(prompt, 0), np.stack([m.hidden(i) for i in range(tokens)])]
+                first = first or got
+                for a, b in zip(first, got):
+                    assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (pdl, int((a != b).any(-1).sum()))
+            m.close()
+    finally:
+        lib.greta_cuda_set_pdl(1)
+
+
 @pytest.mark.parametrize("chunks", [(40, 40), (40, 10), (12, 45, 3)])
 def test_chunked_prefill_attends_to_the_cache(pkg, chunks):
     """A prompt fed in several forward() calls: every chunk after the first starts at pos0 > 0, its queries attend to
