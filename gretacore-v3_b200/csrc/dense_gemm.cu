@@ -152,40 +152,39 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   if (warp == 0) {
     uint32_t issued = 0, s = 0, ph = 1;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
       const int n0 = (int)(t / tok_tiles) * TILE_N, m0 = (int)(t % tok_tiles) * TN;
       for (uint32_t kt = 0; kt < KT; ++kt) {
-        ok = mbar_wait(&empty[s], ph, abort_flag, 100 + s);
-        if (!ok) break;
         uint8_t *st = smem + (size_t)s * C::STAGE;
-        if (leader) {
+        if (ok) ok = mbar_wait(&empty[s], ph, abort_flag, 100 + s);
+        __syncwarp();
+        if (leader && ok) {
           mbar_arrive_expect_tx(&full[s], C::STAGE);
           tma_load_2d(st, &tmap_w, (int)(kt * BK), n0, &full[s]);
           tma_load_2d(st + C::A_BYTES, &tmap_x, (int)(kt * BK), m0, &full[s]);
+          ++issued;
         }
-        ++issued;
         if (++s == ST) {
           s = 0;
           ph ^= 1;
         }
       }
     }
-    if (*abort_flag) drain_copies(full, issued, ST);
+    if (leader && *abort_flag) drain_copies(full, issued, ST);
   } else if (warp == 1) {
     const uint32_t lo0 = smem_desc_lo(smem_u32(smem));
     uint32_t s = 0, ph = 0, it = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, ++it) {
       const uint32_t b = it & 1;
-      ok = mbar_wait(&acc_empty[b], ((it >> 1) & 1) ^ 1, abort_flag, 300 + b);
-      if (!ok) break;
-      tc_fence_after();
+      if (ok) ok = mbar_wait(&acc_empty[b], ((it >> 1) & 1) ^ 1, abort_flag, 300 + b);
+      __syncwarp();
       for (uint32_t kt = 0; kt < KT; ++kt) {
-        ok = mbar_wait(&full[s], ph, abort_flag, 200 + s);
-        if (!ok) break;
-        tc_fence_after();
         const uint32_t w_lo = lo0 + s * (C::STAGE >> 4), x_lo = w_lo + (C::A_BYTES >> 4);
-        if (leader) {
+        if (ok) ok = mbar_wait(&full[s], ph, abort_flag, 200 + s);
+        __syncwarp();
+        if (leader && ok) {
+          tc_fence_after();
 #pragma unroll
           for (int k16 = 0; k16 < BK / 16; ++k16)
             umma_f16(tmem_base + b * TN, w_lo + k16 * 2, x_lo + k16 * 2, SMEM_DESC_HI_SW128, idesc, (kt | k16) ? 1u : 0u);
@@ -196,7 +195,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           ph ^= 1;
         }
       }
-      if (ok && leader) umma_commit(&acc_full[b]);
+      if (leader && ok) umma_commit(&acc_full[b]);
     }
   } else {
     constexpr int SHARE = TN / (C::EPI_WARPS / 4);  // tokens per warp
@@ -235,6 +234,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
   }
   tc_fence_before();
+  __syncwarp();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
@@ -291,31 +291,33 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   const bool leader = elect_one();
   if (warp == 0) {
     uint32_t issued = 0, s = 0, ph = 1;
+    bool ok = true;
     for (uint32_t kt = kt0; kt < kt1; ++kt) {
-      if (!mbar_wait(&empty[s], ph, abort_flag, 100 + s)) break;
       uint8_t *st = smem + (size_t)s * C::STAGE;
-      if (leader) {
+      if (ok) ok = mbar_wait(&empty[s], ph, abort_flag, 100 + s);
+      __syncwarp();
+      if (leader && ok) {
         mbar_arrive_expect_tx(&full[s], C::STAGE);
         tma_load_2d(st, &tmap_w, (int)(kt * BK), (int)n0, &full[s]);
         tma_load_2d(st + C::A_BYTES, &tmap_x, (int)(kt * BK), (int)m0, &full[s]);
+        ++issued;
       }
-      ++issued;
       if (++s == ST) {
         s = 0;
         ph ^= 1;
       }
     }
-    if (*abort_flag) drain_copies(full, issued, ST);
+    if (leader && *abort_flag) drain_copies(full, issued, ST);
   } else if (warp == 1) {
     const uint32_t lo0 = smem_desc_lo(smem_u32(smem));
     uint32_t s = 0, ph = 0;
     bool ok = true;
     for (uint32_t kt = kt0; kt < kt1; ++kt) {
-      ok = mbar_wait(&full[s], ph, abort_flag, 200 + s);
-      if (!ok) break;
-      tc_fence_after();
       const uint32_t w_lo = lo0 + s * (C::STAGE >> 4), x_lo = w_lo + (C::A_BYTES >> 4);
-      if (leader) {
+      if (ok) ok = mbar_wait(&full[s], ph, abort_flag, 200 + s);
+      __syncwarp();
+      if (leader && ok) {
+        tc_fence_after();
 #pragma unroll
         for (int k16 = 0; k16 < BK / 16; ++k16)
           umma_f16(tmem_base, w_lo + k16 * 2, x_lo + k16 * 2, SMEM_DESC_HI_SW128, idesc, (kt > kt0 || k16) ? 1u : 0u);
@@ -326,7 +328,7 @@ linear_tc_split_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         ph ^= 1;
       }
     }
-    if (ok && leader) umma_commit(acc_full);
+    if (leader && ok) umma_commit(acc_full);
   } else {
     constexpr int SHARE = TN / (C::EPI_WARPS / 4);
     const int quad = warp & 3, c_begin = ((warp - 2) >> 2) * SHARE;

@@ -115,39 +115,39 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
     pdl_wait();
     uint32_t s = 0, ph = 1, issued = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < w.tiles && ok; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < w.tiles; t += gridDim.x) {
       const int m0 = (int)((t % w.tok_tiles) * TN);
       for (uint32_t kt = 0; kt < KT; ++kt) {
-        ok = mbar_wait(&act_empty[s], ph, abort_flag, 100 + s);
-        if (!ok) break;
-        if (leader) {
-          uint8_t *dst = act + (size_t)s * act_bytes;
+        uint8_t *dst = act + (size_t)s * act_bytes;
+        if (ok) ok = mbar_wait(&act_empty[s], ph, abort_flag, 100 + s);
+        __syncwarp();
+        if (leader && ok) {
           mbar_arrive_expect_tx(&act_full[s], act_bytes);
           tma_load_2d(dst, &w.act, (int)(kt * TS_K), m0, &act_full[s]);
           tma_load_2d(dst + act_bytes / 2, &w.act, (int)(kt * TS_K + BK), m0, &act_full[s]);
+          ++issued;
         }
-        ++issued;
         if (++s == AS) {
           s = 0;
           ph ^= 1;
         }
       }
     }
-    if (*abort_flag) drain_copies(act_full, issued, AS);
+    if (leader && *abort_flag) drain_copies(act_full, issued, AS);
   } else if (warp == 2) {
-    uint32_t u = 0;
+    uint32_t u = 0, issued = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < w.tiles && ok; t += gridDim.x) {
+    for (uint32_t t = blockIdx.x; t < w.tiles; t += gridDim.x) {
       const uint32_t rt = t / w.tok_tiles, seg = PAIR ? 0u : (rt < w.tile_end[0] ? 0u : (rt < w.tile_end[1] ? 1u : 2u));
       const int n0 = (int)((rt - (seg ? w.tile_end[seg - 1] : 0)) * TILE_ROWS);
       for (uint32_t kq = 0; kq < units; ++kq, ++u) {
         const uint32_t slot = u % TS_RAW_UNITS;
         if (u == TS_RAW_UNITS) pdl_wait();  // from here on the bounded waits depend on the predecessor's end
-        ok = mbar_wait(&raw_empty[slot], ((u / TS_RAW_UNITS) & 1) ^ 1, abort_flag, 200 + slot);
-        if (!ok) break;
-        if (leader) {
-          uint8_t *dst = raw + slot * TS_RAW_BYTES;
-          const int kd = (int)((Q4 ? kq : kq / 2) * 8);  // the scales of 256 elements
+        uint8_t *dst = raw + slot * TS_RAW_BYTES;
+        const int kd = (int)((Q4 ? kq : kq / 2) * 8);  // the scales of 256 elements
+        if (ok) ok = mbar_wait(&raw_empty[slot], ((u / TS_RAW_UNITS) & 1) ^ 1, abort_flag, 200 + slot);
+        __syncwarp();
+        if (leader && ok) {
           mbar_arrive_expect_tx(&raw_full[slot], TS_RAW_BYTES);
           tma_load_2d(dst, &w.qs[seg], (int)(kq * 128), n0, &raw_full[slot]);
           tma_load_2d(dst + TS_RAW_PAYLOAD, &w.d[seg], kd, n0, &raw_full[slot]);
@@ -155,29 +155,26 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
             tma_load_2d(dst + TILE_ROWS * 128, &w.qs[1], (int)(kq * 128), n0, &raw_full[slot]);
             tma_load_2d(dst + TS_RAW_PAYLOAD + TILE_ROWS * 16, &w.d[1], kd, n0, &raw_full[slot]);
           }
+          ++issued;
         }
       }
     }
-    if (*abort_flag) drain_copies(raw_full, u, TS_RAW_UNITS);
+    if (leader && *abort_flag) drain_copies(raw_full, issued, TS_RAW_UNITS);
   } else if (warp == 1) {
     const uint32_t a_lo0 = smem_desc_lo(smem_u32(act)), lg = TS == 4 ? 2 : 1;
     uint32_t s = 0, ph = 0, g = 0, it = 0;
     bool ok = true;
     pdl_wait();
-    for (uint32_t t = blockIdx.x; t < w.tiles && ok; t += gridDim.x, ++it) {
+    for (uint32_t t = blockIdx.x; t < w.tiles; t += gridDim.x, ++it) {
       const uint32_t b = w.accs == 2 ? (it & 1) : 0;
-      ok = mbar_wait(&acc_empty[b], ((w.accs == 2 ? it >> 1 : it) & 1) ^ 1, abort_flag, 300 + b);
-      if (!ok) break;
-      for (uint32_t kt = 0; kt < KT && ok; ++kt) {
-        ok = mbar_wait(&act_full[s], ph, abort_flag, 310 + s);
-        if (!ok) break;
-        const uint32_t a_lo = a_lo0 + s * (act_bytes >> 4), slot = g & (TS - 1);
-        ok = mbar_wait(&w_full[slot], (g >> lg) & 1, abort_flag, 320 + slot);
-        if (!ok) break;
-        ++g;
-        tc_fence_after();
-        if (leader) {
-          const uint32_t d = tmem + b * TN, a = tmem_w + slot * TS_W_COLS;
+      if (ok) ok = mbar_wait(&acc_empty[b], ((w.accs == 2 ? it >> 1 : it) & 1) ^ 1, abort_flag, 300 + b);
+      __syncwarp();
+      for (uint32_t kt = 0; kt < KT; ++kt, ++g) {
+        const uint32_t a_lo = a_lo0 + s * (act_bytes >> 4), slot = g & (TS - 1), d = tmem + b * TN, a = tmem_w + slot * TS_W_COLS;
+        if (ok) ok = mbar_wait(&act_full[s], ph, abort_flag, 310 + s) && mbar_wait(&w_full[slot], (g >> lg) & 1, abort_flag, 320 + slot);
+        __syncwarp();
+        if (leader && ok) {
+          tc_fence_after();
 #pragma unroll
           for (uint32_t k16 = 0; k16 < TS_K / 16; ++k16)
             umma_f16_ts(d, a + k16 * 8, a_lo + (k16 / 4) * (act_bytes >> 5) + (k16 % 4) * 2, SMEM_DESC_HI_SW128, w.idesc, (kt | k16) ? 1u : 0u);
@@ -189,7 +186,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
           ph ^= 1;
         }
       }
-      if (ok && leader) umma_commit(&acc_full[b]);
+      if (leader && ok) umma_commit(&acc_full[b]);
     }
   } else if (warp >= (int)TS_DEQ_WARP0 && warp < (int)TS_EPI_WARP0) {
     // The set of a stage is its weight slot, and with whole units in every tile a raw slot is always read by the same sets: whoever waits on
@@ -341,6 +338,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_ts_kernel(const __grid_con
     }
   }
   tc_fence_before();
+  __syncwarp();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
