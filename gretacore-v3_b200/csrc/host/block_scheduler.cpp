@@ -56,6 +56,7 @@ TensorShard tensor_shard(const ModelConfig &c, LayerTensor t) {
 }
 
 namespace {
+constexpr size_t SKINNY_ROWS = 32;  // prompt rows up to which the projections are GEMVs on fp32 activations
 struct PlanePair {
   Buffer *qs, *d;
 };
@@ -166,11 +167,12 @@ bool BlockScheduler::allocate_activations(size_t batch_size, size_t max_seq_len,
   cur_seq_ = 0;
   if (c.arch == ModelArch::HYBRID) return allocate_hybrid_activations(err);
   const size_t S = std::max(max_seq_len, batch_size), D = c.dim, B = batch_size;
+  const size_t few = std::min<size_t>(S, SKINNY_ROWS);  // rows of what the route for more rows has no use for
   const size_t ql = (size_t)heads_l_ * c.head_dim, kvl = (size_t)kv_heads_l_ * c.head_dim;
   auto dev = [&](Buffer &b, size_t bytes, GretaDataType t = GretaDataType::FP32) { return b.allocate(bytes, BufferUsage::DeviceOnly, t, err); };
   ActivationBuffers &a = activations_;
   if (!dev(a.x, S * D * 4) || !dev(a.norm_out, S * D * 4) || !dev(a.q, S * ql * 4) || !dev(a.k, S * kvl * 4) || !dev(a.v, S * kvl * 4) ||
-      !dev(a.attn_out, S * ql * 4) || !dev(a.mlp_gate, S * hidden_l_ * 4) || !dev(a.mlp_up, S * hidden_l_ * 4) || !dev(a.mlp_out, S * D * 4))
+      !dev(a.attn_out, S * ql * 4) || !dev(a.mlp_gate, S * hidden_l_ * 4) || !dev(a.mlp_up, few * hidden_l_ * 4) || !dev(a.mlp_out, (c.tp_size > 1 ? S : few) * D * 4))
     return false;
   const size_t cache = (size_t)c.num_layers * B * kv_heads_l_ * max_seq_len * c.head_dim * 2;  // [L][B][Hkv][S][Dh] fp16
   if (!dev(a.kv_cache_k, cache, GretaDataType::FP16) || !dev(a.kv_cache_v, cache, GretaDataType::FP16)) return false;
@@ -179,7 +181,6 @@ bool BlockScheduler::allocate_activations(size_t batch_size, size_t max_seq_len,
       !dev(a.out_tokens, B * max_seq_len * 4))
     return false;
   if (!dev(a.attn_scratch, greta_cuda_attn_decode_scratch_bytes((uint32_t)B * heads_l_, c.head_dim))) return false;
-  if (!dev(a.gemm_ws, greta_cuda_gemm_workspace_bytes((uint32_t)max_seq_len, std::max(c.dim, c.hidden_dim)))) return false;
   if (!dev(logits_, B * (size_t)c.vocab_size * 4)) return false;
   if (B > 1 && c.tp_size > 1 && !dev(logits_local_, B * (size_t)vocab_l_ * 4)) return false;
   if (B > 1 && !dev(batch_ws_, greta_cuda_gemv_batch_workspace_bytes((uint32_t)B, std::max({c.dim, (uint32_t)ql, hidden_l_})))) return false;
@@ -579,8 +580,7 @@ bool BlockScheduler::lm_head_batch(std::string *err) {
 
 bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t seq_len, const int32_t *, std::string *err) {
   // Prefill form of one layer over S = seq_len rows (the reference's operator order,
-  // block_scheduler.cpp:1814-3032), projections through GretaCompute-style routing: GEMV for
-  // S <= 32, tensor-core GEMM above.
+  // block_scheduler.cpp:1814-3032): up to 32 rows by fp32 activations and the GEMVs, operator by operator, above on the tensor cores.
   const ModelConfig &c = config_;
   ActivationBuffers &a = activations_;
   if (layer_idx >= blocks_.size()) return fail(err, "execute_layer: layer out of range");
@@ -598,10 +598,9 @@ bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t se
   float *att = static_cast<float *>(a.attn_out.data()), *gate = static_cast<float *>(a.mlp_gate.data()), *up = static_cast<float *>(a.mlp_up.data());
   float *tmp = static_cast<float *>(a.mlp_out.data());
   const bool tp = c.tp_size > 1;
-  // Prompts: products that share their activations in one launch, operands rounded to fp16 where they are made, SwiGLU and residual
-  // in the products' epilogues.  The same roundings as the operator-by-operator form below, which keeps up to 32 rows, other formats and
-  // head sizes.
-  if (S > 32 && (fmt == GRETA_FMT_Q4_0 || fmt == GRETA_FMT_Q8_0) && Dh % 8 == 0 && Dh <= 1024) {
+  // More than 32 rows: products that share their activations in one launch, operands rounded to fp16 where they are made, SwiGLU and residual
+  // in the products' epilogues.
+  if (S > SKINNY_ROWS) {
     void *n16 = a.norm_out.data(), *gate16 = a.mlp_gate.data();  // fp16 rows in buffers sized for fp32
     const greta_gemm_segment qkv[3] = {{b.wq.data(), b.s_wq.data(), ql, q}, {b.wk.data(), b.s_wk.data(), kvl, k}, {b.wv.data(), b.s_wv.data(), kvl, v}};
     const greta_gemm_segment ffn[2] = {{b.w1.data(), b.s_w1.data(), hidden_l_, gate16}, {b.w3.data(), b.s_w3.data(), hidden_l_, nullptr}};
@@ -624,8 +623,7 @@ bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t se
     return residual(gate16, b.w2, b.s_w2, hidden_l_, "w2");
   }
   auto proj = [&](const float *in, Buffer &w, Buffer &sw, float *out, uint32_t N, uint32_t K) -> int {
-    if (S <= 32) return greta_cuda_gemv(s, fmt, in, 0, w.data(), sw.data(), out, S, N, K);
-    return greta_cuda_gemm(s, fmt, in, 0, w.data(), sw.data(), out, 0, S, N, K, a.gemm_ws.data());
+    return greta_cuda_gemv(s, fmt, in, 0, w.data(), sw.data(), out, S, N, K);
   };
   GRETA_TRY(greta_cuda_rmsnorm(s, x, static_cast<const float *>(b.attn_norm.data()), nrm, S, D, c.rms_eps), "rmsnorm");
   GRETA_TRY(proj(nrm, b.wq, b.s_wq, q, ql, D), "wq");

@@ -549,7 +549,7 @@ struct BlockBuffers {
 struct ActivationBuffers {
   gcore::rt::cuda::Buffer x, q, k, v, attn_out, mlp_gate, mlp_up, mlp_out, norm_out;
   gcore::rt::cuda::Buffer kv_cache_k, kv_cache_v;   // fp16 [L][Hkv_local][max_seq][Dh]
-  gcore::rt::cuda::Buffer tokens, d_pos, d_next, attn_scratch, gemm_ws, out_tokens;
+  gcore::rt::cuda::Buffer tokens, d_pos, d_next, attn_scratch, out_tokens;
 };
 
 // One layer of a hybrid design: everything of the mixer that reads the norm's output packed in one weight (w_in), its output

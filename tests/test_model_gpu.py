@@ -1,6 +1,8 @@
 """Model-level parity: logits and greedy token ids of the C++ host layer (BlockScheduler / Generator
 on the CUDA kernels) against the CPU oracle, on a small Llama-shaped model with seeded synthetic
 weights.  Token ids must be identical; logits within the matmul tolerance."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -114,6 +116,28 @@ def test_whole_prompts_give_the_same_bits_every_time(pkg, tokens, fmt_name):
             m.close()
     finally:
         lib.greta_cuda_set_pdl(1)
+
+
+def test_prompt_buffers_are_those_that_the_route_uses(pkg):
+    """The feed-forward's fp32 `up` rows and the products' workspace belong to routes that a long prompt does not take: only `gate` is held for every row."""
+    pkg.ffi.cuda()
+    cudart = C.CDLL("libcudart.so.12")   # the one that the library is linked to
+
+    def free_bytes():
+        free, total = C.c_size_t(), C.c_size_t()
+        assert cudart.cudaMemGetInfo(C.byref(free), C.byref(total)) == 0
+        return free.value
+
+    cfg = dict(SMALL, hidden_dim=8192, max_seq=8192)
+    S, D, ql, kvl = cfg["max_seq"], cfg["dim"], 256, 128
+    pkg.model.Model(cfg).close()         # what the process holds once
+    before = free_bytes()
+    m = pkg.model.Model(cfg)
+    held = before - free_bytes()
+    weights = 2 * (2 * D * ql + 2 * D * kvl + 3 * D * cfg["hidden_dim"]) * 18 // 32 + 4 * cfg["vocab"] * D
+    rows = 4 * S * (cfg["hidden_dim"] + 2 * D + 2 * ql + 2 * kvl) + 2 * 2 * S * kvl * 2
+    assert held < weights + rows + (100 << 20), held   # 100 MB: allocation granularity and small buffers; `up` alone would be 268
+    m.close()
 
 
 @pytest.mark.parametrize("chunks", [(40, 40), (40, 10), (12, 45, 3)])
