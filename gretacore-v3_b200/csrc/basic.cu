@@ -108,14 +108,19 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ 
 
 // The same values as fp16, for the tensor-core products.  A row stays in registers (PER values per thread, all loads under way together;
 // the 256-thread order of the sum is rmsnorm_kernel's, so the results are its bits): 3.8 us for 512 x 4096 in the layer against 10.8 and a
-// conversion pass of 2.9 per product.
+// conversion pass of 2.9 per product.  y32 may be null; otherwise it takes the fp32 values as well.
 template <int PER>
-__global__ void __launch_bounds__(256) rmsnorm_f16_kernel(const float *x, const float *__restrict__ gamma, __half *y, uint32_t cols, float eps) {
+__global__ void __launch_bounds__(256) rmsnorm_f16_kernel(const float *x, const float *__restrict__ gamma, __half *y, float *y32, uint32_t cols, float eps) {
   __shared__ float sm[32];
   pdl_launch_dependents();
   pdl_wait();
   const float *xr = x + (size_t)blockIdx.x * cols;
   __half *yr = y + (size_t)blockIdx.x * cols;
+  float *y32r = y32 ? y32 + (size_t)blockIdx.x * cols : nullptr;
+  auto put = [&](uint32_t c, float n) {
+    yr[c] = __float2half_rn(n);
+    if (y32r) y32r[c] = n;
+  };
   float v[PER], ss = 0.f;
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
@@ -130,9 +135,9 @@ __global__ void __launch_bounds__(256) rmsnorm_f16_kernel(const float *x, const 
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     const uint32_t c = threadIdx.x + i * 256;
-    if (c < cols) yr[c] = __float2half_rn((v[i] * inv) * gamma[c]);
+    if (c < cols) put(c, (v[i] * inv) * gamma[c]);
   }
-  for (uint32_t c = threadIdx.x + PER * 256; c < cols; c += 256) yr[c] = __float2half_rn((xr[c] * inv) * gamma[c]);
+  for (uint32_t c = threadIdx.x + PER * 256; c < cols; c += 256) put(c, (xr[c] * inv) * gamma[c]);
 }
 
 __global__ void add_kernel(const float *a, const float *b, float *c, size_t n) {
@@ -277,6 +282,12 @@ int launch_argmax(cudaStream_t stream, const float *logits, uint32_t n, uint32_t
   return launched("argmax_kernel");
 }
 
+int launch_rmsnorm_f16(cudaStream_t stream, const float *x, const float *gamma, void *y, float *y32, uint32_t rows, uint32_t cols, float eps) {
+  auto go = [&](auto kernel) { return launch_pdl(kernel, dim3(rows), dim3(256), 0, stream, x, gamma, static_cast<__half *>(y), y32, cols, eps); };
+  GRETA_CUDA_TRY(cols <= 256 * 8 ? go(rmsnorm_f16_kernel<8>) : cols <= 256 * 16 ? go(rmsnorm_f16_kernel<16>) : go(rmsnorm_f16_kernel<32>));
+  return launched("rmsnorm_f16_kernel");
+}
+
 inline unsigned blocks_for(size_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -347,14 +358,12 @@ int greta_cuda_rmsnorm(greta_stream_t stream, const float *x, const float *gamma
 int greta_cuda_rmsnorm_f16(greta_stream_t stream, const float *x, const float *gamma, void *y, uint32_t rows, uint32_t cols, float eps) {
   if (rows == 0 || cols == 0) return GRETA_OK;
   GRETA_REQUIRE(x && gamma && y, "rmsnorm_f16: null pointer");
-  __half *y16 = static_cast<__half *>(y);
-  if (cols <= 256 * 8)
-    GRETA_CUDA_TRY(launch_pdl(rmsnorm_f16_kernel<8>, dim3(rows), dim3(256), 0, S(stream), x, gamma, y16, cols, eps));
-  else if (cols <= 256 * 16)
-    GRETA_CUDA_TRY(launch_pdl(rmsnorm_f16_kernel<16>, dim3(rows), dim3(256), 0, S(stream), x, gamma, y16, cols, eps));
-  else
-    GRETA_CUDA_TRY(launch_pdl(rmsnorm_f16_kernel<32>, dim3(rows), dim3(256), 0, S(stream), x, gamma, y16, cols, eps));
-  return launched("rmsnorm_f16_kernel");
+  return launch_rmsnorm_f16(S(stream), x, gamma, y, nullptr, rows, cols, eps);
+}
+int greta_cuda_rmsnorm_both(greta_stream_t stream, const float *x, const float *gamma, float *y, void *y_f16, uint32_t rows, uint32_t cols, float eps) {
+  if (rows == 0 || cols == 0) return GRETA_OK;
+  GRETA_REQUIRE(x && gamma && y && y_f16, "rmsnorm_both: null pointer");
+  return launch_rmsnorm_f16(S(stream), x, gamma, y_f16, y, rows, cols, eps);
 }
 int greta_cuda_add(greta_stream_t stream, const float *a, const float *b, float *c, size_t n) {
   if (n == 0) return GRETA_OK;

@@ -174,6 +174,7 @@ bool BlockScheduler::allocate_activations(size_t batch_size, size_t max_seq_len,
   if (!dev(a.x, S * D * 4) || !dev(a.norm_out, S * D * 4) || !dev(a.q, S * ql * 4) || !dev(a.k, S * kvl * 4) || !dev(a.v, S * kvl * 4) ||
       !dev(a.attn_out, S * ql * 4) || !dev(a.mlp_gate, S * hidden_l_ * 4) || !dev(a.mlp_up, few * hidden_l_ * 4) || !dev(a.mlp_out, (c.tp_size > 1 ? S : few) * D * 4))
     return false;
+  if (S > SKINNY_ROWS && !dev(a.norm_f16, S * D * 2, GretaDataType::FP16)) return false;
   const size_t cache = (size_t)c.num_layers * B * kv_heads_l_ * max_seq_len * c.head_dim * 2;  // [L][B][Hkv][S][Dh] fp16
   if (!dev(a.kv_cache_k, cache, GretaDataType::FP16) || !dev(a.kv_cache_v, cache, GretaDataType::FP16)) return false;
   // d_pos: B positions, then B counts of ids produced; d_next: B token ids; out_tokens: [B][max_seq]
@@ -579,6 +580,10 @@ bool BlockScheduler::lm_head_batch(std::string *err) {
 }
 
 bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t seq_len, const int32_t *, std::string *err) {
+  return prompt_layer(layer_idx, seq_start, seq_len, true, err);
+}
+
+bool BlockScheduler::prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err) {
   // Prefill form of one layer over S = seq_len rows (the reference's operator order,
   // block_scheduler.cpp:1814-3032): up to 32 rows by fp32 activations and the GEMVs, operator by operator, above on the tensor cores.
   const ModelConfig &c = config_;
@@ -601,7 +606,7 @@ bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t se
   // More than 32 rows: products that share their activations in one launch, operands rounded to fp16 where they are made, SwiGLU and residual
   // in the products' epilogues.
   if (S > SKINNY_ROWS) {
-    void *n16 = a.norm_out.data(), *gate16 = a.mlp_gate.data();  // fp16 rows in buffers sized for fp32
+    void *n16 = a.norm_f16.data(), *gate16 = a.mlp_gate.data();  // gate: fp16 rows in a buffer sized for fp32
     const greta_gemm_segment qkv[3] = {{b.wq.data(), b.s_wq.data(), ql, q}, {b.wk.data(), b.s_wk.data(), kvl, k}, {b.wv.data(), b.s_wv.data(), kvl, v}};
     const greta_gemm_segment ffn[2] = {{b.w1.data(), b.s_w1.data(), hidden_l_, gate16}, {b.w3.data(), b.s_w3.data(), hidden_l_, nullptr}};
     auto residual = [&](const void *in, Buffer &w, Buffer &sw, uint32_t K, const char *name) -> bool {
@@ -618,7 +623,9 @@ bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t se
     GRETA_TRY(greta_cuda_attn_prefill(s, q, kc, vc, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
     GRETA_TRY(greta_cuda_f32_to_f16(s, att, q, (size_t)S * ql), "attention output");  // the queries are done with
     if (!residual(q, b.wo, b.s_wo, ql, "wo")) return false;
-    GRETA_TRY(greta_cuda_rmsnorm_f16(s, x, static_cast<const float *>(b.ffn_norm.data()), n16, S, D, c.rms_eps), "rmsnorm");
+    const float *gamma = static_cast<const float *>(b.ffn_norm.data());
+    GRETA_TRY(keep_norm ? greta_cuda_rmsnorm_both(s, x, gamma, nrm, n16, S, D, c.rms_eps) : greta_cuda_rmsnorm_f16(s, x, gamma, n16, S, D, c.rms_eps),
+              "rmsnorm");
     GRETA_TRY(greta_cuda_gemm_segments(s, fmt, n16, S, D, ffn, 2, GRETA_GEMM_SWIGLU_F16), "w1, w3");
     return residual(gate16, b.w2, b.s_w2, hidden_l_, "w2");
   }
@@ -673,7 +680,7 @@ bool BlockScheduler::forward(const int32_t *tokens, size_t seq_start, size_t seq
     if (!decode_layers(err)) return false;
   } else {  // prefill form, on the current sequence's cache (also a single token when the scheduler holds a batch)
     for (size_t l = 0; l < blocks_.size(); ++l)
-      if (!execute_layer(l, seq_start, seq_len, tokens, err)) return false;
+      if (!prompt_layer(l, seq_start, seq_len, l + 1 == blocks_.size(), err)) return false;
   }
   if (!lm_head(static_cast<const float *>(a.x.data()) + (seq_len - 1) * c.dim, err)) return false;
   GRETA_TRY(greta_cuda_stream_synchronize(s), "forward");

@@ -548,6 +548,7 @@ struct BlockBuffers {
 
 struct ActivationBuffers {
   gcore::rt::cuda::Buffer x, q, k, v, attn_out, mlp_gate, mlp_up, mlp_out, norm_out;
+  gcore::rt::cuda::Buffer norm_f16;                 // norm rows as the prompt's products read them
   gcore::rt::cuda::Buffer kv_cache_k, kv_cache_v;   // fp16 [L][Hkv_local][max_seq][Dh]
   gcore::rt::cuda::Buffer tokens, d_pos, d_next, attn_scratch, out_tokens;
 };
@@ -621,7 +622,7 @@ public:
   bool decode_step_host(const int32_t *pinned_token_in, int32_t *pinned_token_out, std::string *err);
 
   gcore::rt::cuda::Buffer &get_hidden_state() { return activations_.x; }
-  gcore::rt::cuda::Buffer &get_norm_out() { return activations_.norm_out; }
+  gcore::rt::cuda::Buffer &get_norm_out() { return activations_.norm_out; }  // fp32 rows of the last layer's feed-forward norm
   const gcore::rt::cuda::Buffer &get_logits() const { return logits_; }
   const gcore::rt::cuda::Buffer &get_output_weight() const { return output_weight_; }
   const ModelConfig &config() const { return config_; }
@@ -640,6 +641,7 @@ private:
   bool decode_layers_batch(std::string *err);
   bool lm_head_batch(std::string *err);
   bool step_fits(std::string *err) const;
+  bool prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err);  // keep_norm: norm_out is filled
   void invalidate_graph();
   bool build_decode_plan(std::string *err);
   bool lm_head(const float *x_row, std::string *err);

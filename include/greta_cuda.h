@@ -413,6 +413,9 @@ GRETA_API int greta_cuda_rmsnorm(greta_stream_t stream, const float *x, const fl
                                  uint32_t rows, uint32_t cols, float eps);
 /* The same, rounded to fp16. */
 GRETA_API int greta_cuda_rmsnorm_f16(greta_stream_t stream, const float *x, const float *gamma, void *y, uint32_t rows, uint32_t cols, float eps);
+/* Both of them in one launch: fp32 to y, fp16 to y_f16. */
+GRETA_API int greta_cuda_rmsnorm_both(greta_stream_t stream, const float *x, const float *gamma, float *y, void *y_f16, uint32_t rows, uint32_t cols,
+                                      float eps);
 /* launch_add (basic_kernels.hip:127-140). */
 GRETA_API int greta_cuda_add(greta_stream_t stream, const float *a, const float *b, float *c, size_t n);
 /* launch_silu, launch_mul (basic_kernels.hip:141-167), separately. */

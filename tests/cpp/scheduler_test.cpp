@@ -1,0 +1,83 @@
+// Drives BlockScheduler from C++ where the C interface does not reach: buffers that it exposes and the tensor-parallel hooks.  The first
+// argument names the check; exits non-zero when it fails.  Built by gretacore-v3_b200/csrc/Makefile (target scheduler_test) and run by
+// tests/test_scheduler_gpu.py.
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "gcore/inference/block_scheduler.hpp"
+
+using namespace gcore::inference;
+using gcore::rt::GretaDataType;
+
+static std::string g_err;
+static int complain(const std::string &what) {
+  fprintf(stderr, "%s: %s\n", what.c_str(), g_err.c_str());
+  return 1;
+}
+
+static ModelConfig small() {
+  ModelConfig c;
+  c.dim = 512; c.num_heads = 8; c.num_heads_kv = 4; c.num_layers = 2; c.vocab_size = 1000; c.hidden_dim = 1536; c.head_dim = 64; c.max_seq_len = 160;
+  c.rope_base = 10000.0f; c.rms_eps = 1e-5f;
+  c.weight_type = GretaDataType::Q4_0; c.lm_head_type = GretaDataType::FP16;
+  return c;
+}
+static std::vector<int32_t> prompt(size_t n) {
+  std::vector<int32_t> t(n);
+  for (size_t i = 0; i < n; ++i) t[i] = (int32_t)((i * 7919 + 13) % 1000);
+  return t;
+}
+static bool start(BlockScheduler &s, const ModelConfig &c) {
+  return s.init(c, &g_err) && s.allocate_weights(&g_err) && s.load_synthetic_weights(5, &g_err) && s.allocate_activations(1, c.max_seq_len, &g_err);
+}
+static std::vector<float> rows_of(gcore::rt::cuda::Buffer &b, size_t n) {
+  std::vector<float> v(n);
+  if (!b.copy_to_host(v.data(), n * 4, &g_err)) v.clear();
+  return v;
+}
+
+// get_norm_out() after a prompt: fp32 rows of the last layer's feed-forward norm, on either side of 32 rows, after forward() and after
+// execute_layer().  With a norm weight of one a row's root mean square is one.
+static int norm_out() {
+  const ModelConfig c = small();
+  BlockScheduler s;
+  if (!start(s, c)) return complain("start");
+  std::vector<float> ones(c.dim, 1.0f);
+  for (size_t l = 0; l < c.num_layers; ++l)
+    if (!s.set_layer_tensor(l, LayerTensor::FFN_NORM, ones.data(), ones.size() * 4, &g_err)) return complain("set_layer_tensor");
+  const std::vector<int32_t> t = prompt(150);
+  std::vector<float> few;
+  for (size_t n : {(size_t)32, (size_t)33, (size_t)150}) {
+    for (int layer = -1; layer < 1; ++layer) {
+      if (!s.forward(t.data(), 0, n, &g_err)) return complain("forward");
+      if (layer >= 0 && (!s.execute_layer(layer, 0, n, t.data(), &g_err) || !s.stream() || (s.stream()->synchronize(), false))) return complain("execute_layer");
+      const std::vector<float> v = rows_of(s.get_norm_out(), n * c.dim);
+      if (v.empty()) return complain("get_norm_out");
+      for (size_t r = 0; r < n; ++r) {
+        double ss = 0;
+        for (size_t i = 0; i < c.dim; ++i) ss += (double)v[r * c.dim + i] * v[r * c.dim + i];
+        if (!(std::fabs(std::sqrt(ss / c.dim) - 1) < 1e-2)) {
+          fprintf(stderr, "%zu rows, layer %d: row %zu has rms %g\n", n, layer, r, std::sqrt(ss / c.dim));
+          return 1;
+        }
+      }
+      if (layer < 0 && n == 32) few = v;
+      if (layer < 0 && n > 32) {  // the same rows through fp16 products
+        double worst = 0;
+        for (size_t i = 0; i < few.size(); ++i) worst = std::fmax(worst, std::fabs((double)few[i] - v[i]));
+        if (!(worst < 2e-2)) return fprintf(stderr, "%zu rows differ from 32 by %g\n", n, worst), 1;
+      }
+    }
+  }
+  return 0;
+}
+
+int main(int argc, char **argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  const int rc = what == "norm_out" ? norm_out() : 2;
+  printf("%s: %s\n", what.c_str(), rc ? "FAIL" : "PASS");
+  return rc;
+}

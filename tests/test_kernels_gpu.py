@@ -864,3 +864,16 @@ def test_prefill_fused_elementwise(g, S, H, Hkv, Dh, pos):
         g.check(lib.greta_cuda_f32_to_f16(None, y.ptr, h.ptr, 3 * cols))
         g.check(lib.greta_cuda_rmsnorm_f16(None, dx.ptr, dg.ptr, h2.ptr, 3, cols, 1e-5))
         assert (h.download(np.uint16)[:3 * cols] == h2.download(np.uint16)[:3 * cols]).all()
+
+
+@pytest.mark.parametrize("cols", [7, 2048, 4097, 9000])
+def test_rmsnorm_both(g, cols):
+    """fp32 and fp16 rows of one launch: the bits of the two operators."""
+    rng, lib = np.random.default_rng(cols), g.cuda()
+    x, gm = rng.normal(0, 3, (3, cols)).astype(np.float32), rng.normal(1, 0.1, cols).astype(np.float32)
+    dx, dg, y, h, y2, h2 = _dev(g, x), _dev(g, gm), _dev(g, x), _dev(g, x), _dev(g, x), _dev(g, x)
+    g.check(lib.greta_cuda_rmsnorm(None, dx.ptr, dg.ptr, y.ptr, 3, cols, 1e-5))
+    g.check(lib.greta_cuda_rmsnorm_f16(None, dx.ptr, dg.ptr, h.ptr, 3, cols, 1e-5))
+    g.check(lib.greta_cuda_rmsnorm_both(None, dx.ptr, dg.ptr, y2.ptr, h2.ptr, 3, cols, 1e-5))
+    assert (y.download(np.uint32) == y2.download(np.uint32)).all()
+    assert (h.download(np.uint16)[:3 * cols] == h2.download(np.uint16)[:3 * cols]).all()
