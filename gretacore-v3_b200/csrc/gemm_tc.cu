@@ -35,6 +35,7 @@ using namespace greta;
 
 namespace greta {
 int gemm_ts_status(int *code);  // gemm_ts.cu
+int gemm_ts_set_status(int code);
 }
 
 namespace {
@@ -1125,6 +1126,11 @@ int greta_cuda_gemm_status(int *code) {
   GRETA_REQUIRE(code, "gemm_status: null out pointer");
   GRETA_CUDA_TRY(cudaMemcpyFromSymbol(code, g_gemm_error, sizeof(int)));
   return *code ? GRETA_OK : gemm_ts_status(code);
+}
+
+int greta_cuda_gemm_set_status(int code) {
+  GRETA_CUDA_TRY(cudaMemcpyToSymbol(g_gemm_error, &code, sizeof(int)));
+  return gemm_ts_set_status(code);
 }
 
 int greta_cuda_gemm(greta_stream_t stream, int fmt, const void *A, int a_is_f16, const void *qs, const void *d, void *Cout, int c_is_f16,

@@ -387,7 +387,17 @@ int gemm_ts_status(int *code) {
   GRETA_CUDA_TRY(cudaMemcpyFromSymbol(code, g_gemm_error, sizeof(int)));
   return GRETA_OK;
 }
+int gemm_ts_set_status(int code) {
+  GRETA_CUDA_TRY(cudaMemcpyToSymbol(g_gemm_error, &code, sizeof(int)));
+  return GRETA_OK;
+}
 }  // namespace greta
+
+extern "C" int greta_cuda_gemm_segments_status(greta_stream_t stream, int *code) {
+  GRETA_REQUIRE(code, "gemm_segments_status: null out pointer");
+  GRETA_CUDA_TRY(cudaMemcpyFromSymbolAsync(code, g_gemm_error, sizeof(int), 0, cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  return GRETA_OK;
+}
 
 extern "C" int greta_cuda_gemm_segments(greta_stream_t stream, int fmt, const void *a_f16, uint32_t M, uint32_t K, const greta_gemm_segment *segs,
                                         uint32_t n_segs, int mode) {

@@ -174,7 +174,7 @@ bool BlockScheduler::allocate_activations(size_t batch_size, size_t max_seq_len,
   if (!dev(a.x, S * D * 4) || !dev(a.norm_out, S * D * 4) || !dev(a.q, S * ql * 4) || !dev(a.k, S * kvl * 4) || !dev(a.v, S * kvl * 4) ||
       !dev(a.attn_out, S * ql * 4) || !dev(a.mlp_gate, S * hidden_l_ * 4) || !dev(a.mlp_up, few * hidden_l_ * 4) || !dev(a.mlp_out, (c.tp_size > 1 ? S : few) * D * 4))
     return false;
-  if (S > SKINNY_ROWS && !dev(a.norm_f16, S * D * 2, GretaDataType::FP16)) return false;
+  if (S > SKINNY_ROWS && (!dev(a.norm_f16, S * D * 2, GretaDataType::FP16) || !a.gave_up.allocate(16, BufferUsage::HostVisible, GretaDataType::FP32, err))) return false;
   const size_t cache = (size_t)c.num_layers * B * kv_heads_l_ * max_seq_len * c.head_dim * 2;  // [L][B][Hkv][S][Dh] fp16
   if (!dev(a.kv_cache_k, cache, GretaDataType::FP16) || !dev(a.kv_cache_v, cache, GretaDataType::FP16)) return false;
   // d_pos: B positions, then B counts of ids produced; d_next: B token ids; out_tokens: [B][max_seq]
@@ -683,7 +683,14 @@ bool BlockScheduler::forward(const int32_t *tokens, size_t seq_start, size_t seq
       if (!prompt_layer(l, seq_start, seq_len, l + 1 == blocks_.size(), err)) return false;
   }
   if (!lm_head(static_cast<const float *>(a.x.data()) + (seq_len - 1) * c.dim, err)) return false;
+  int *gave_up = seq_len > SKINNY_ROWS ? static_cast<int *>(a.gave_up.data()) : nullptr;
+  if (gave_up) GRETA_TRY(greta_cuda_gemm_segments_status(s, gave_up), "forward");
   GRETA_TRY(greta_cuda_stream_synchronize(s), "forward");
+  if (gave_up && *gave_up) {  // results and cache rows are wrong; the code is reported once
+    const int code = *gave_up;
+    greta_cuda_gemm_set_status(0);
+    return fail(err, "forward: a bounded wait of a prompt product gave up (code " + std::to_string(code) + ")");
+  }
   return true;
 }
 

@@ -548,6 +548,7 @@ struct BlockBuffers {
 
 struct ActivationBuffers {
   gcore::rt::cuda::Buffer x, q, k, v, attn_out, mlp_gate, mlp_up, mlp_out, norm_out;
+  gcore::rt::cuda::Buffer gave_up;                  // page-locked: code of a wait of the prompt's products that gave up, 0 if none did
   gcore::rt::cuda::Buffer norm_f16;                 // norm rows as the prompt's products read them
   gcore::rt::cuda::Buffer kv_cache_k, kv_cache_v;   // fp16 [L][Hkv_local][max_seq][Dh]
   gcore::rt::cuda::Buffer tokens, d_pos, d_next, attn_scratch, out_tokens;

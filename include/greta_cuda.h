@@ -309,6 +309,8 @@ GRETA_API int greta_cuda_gemm_route(uint32_t M, uint32_t N, uint32_t K, int has_
  * memory and records a non-zero code (100 * role + stage) that this call returns in *code (0 = none).
  * Synchronises with the device. */
 GRETA_API int greta_cuda_gemm_status(int *code);
+/* What greta_cuda_gemm_status reports from here on, until a wait gives up: 0 clears a code that has been dealt with. */
+GRETA_API int greta_cuda_gemm_set_status(int code);
 GRETA_API int greta_cuda_gemm(greta_stream_t stream, int fmt, const void *A, int a_is_f16,
                               const void *qs, const void *d, void *C, int c_is_f16, uint32_t M,
                               uint32_t N, uint32_t K, void *workspace);
@@ -326,6 +328,8 @@ typedef struct greta_gemm_segment {
 } greta_gemm_segment;
 GRETA_API int greta_cuda_gemm_segments(greta_stream_t stream, int fmt, const void *a_f16, uint32_t M, uint32_t K, const greta_gemm_segment *segs,
                                        uint32_t n_segs, int mode);
+/* The code of its kernels so far on the stream: valid in *code once the stream has been synchronised (*code in page-locked memory). */
+GRETA_API int greta_cuda_gemm_segments_status(greta_stream_t stream, int *code);
 
 /* ------------------------------------------------------------------ attention
  * Decode attention of one query per head over the fp16 KV cache

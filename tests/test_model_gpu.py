@@ -140,6 +140,24 @@ def test_prompt_buffers_are_those_that_the_route_uses(pkg):
     m.close()
 
 
+def test_forward_reports_a_product_that_gave_up(pkg):
+    """A bounded wait that gave up in a prompt's products leaves a code on the device; forward() fails with it, once, and the next prompt is as before.
+    The code is written by the host here."""
+    lib, code = pkg.ffi.cuda(), C.c_int(-1)
+    m = pkg.model.Model(SMALL)
+    m.load_synthetic(4)
+    prompt = pkg.model.synth_tokens(4, 40, SMALL["vocab"])
+    first = m.forward(prompt, 0)
+    pkg.ffi.check(lib.greta_cuda_gemm_set_status(123))
+    assert lib.greta_cuda_gemm_status(C.byref(code)) == 0 and code.value == 123
+    m.forward(prompt[:32], 0)                            # no product of that kind in it
+    with pytest.raises(RuntimeError, match="gave up.*123"):
+        m.forward(prompt, 0)
+    assert lib.greta_cuda_gemm_status(C.byref(code)) == 0 and code.value == 0
+    assert np.array_equal(m.forward(prompt, 0), first)
+    m.close()
+
+
 @pytest.mark.parametrize("chunks", [(40, 40), (40, 10), (12, 45, 3)])
 def test_chunked_prefill_attends_to_the_cache(pkg, chunks):
     """A prompt fed in several forward() calls: every chunk after the first starts at pos0 > 0, its queries attend to
