@@ -903,10 +903,8 @@ bool BlockScheduler::decode_step_host(const int32_t *token_in, int32_t *token_ou
 bool BlockScheduler::read_generated(int32_t *out, size_t n, std::string *err) {
   GRETA_TRY(greta_cuda_stream_synchronize(H(stream_)), "read_generated");
   if (n > decode_steps_) return fail(err, "read_generated: fewer steps were run");
-  if (n == 0) return true;
   // out is [batch][n]; the device list is [batch][max_seq].  One strided copy: a copy per sequence cost 7 us each.
-  GRETA_TRY(greta_cuda_memcpy_2d_d2h_sync(out, n * 4, activations_.out_tokens.data(), (size_t)max_seq_ * 4, n * 4, batch_), "read_generated");
-  return true;
+  return activations_.out_tokens.copy_rows_to_host(out, (size_t)max_seq_ * 4, n * 4, batch_, err);
 }
 
 // ------------------------------------------------------------------ Generator

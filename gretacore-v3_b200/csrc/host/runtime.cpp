@@ -64,6 +64,19 @@ bool Buffer::copy_to_host_offset(void *host_ptr, size_t offset, size_t size, std
   return true;
 }
 
+bool Buffer::copy_rows_to_host(void *host_ptr, size_t pitch, size_t width, size_t rows, std::string *err) const {
+  if (!ptr_ || (rows && (rows - 1) * pitch + width > size_))
+    return host::fail(err, "Buffer copy out of bounds: " + std::to_string(rows) + " rows of " + std::to_string(width) + ", pitch=" + std::to_string(pitch) +
+                               ", total_size=" + std::to_string(size_));
+  if (rows == 0 || width == 0) return true;
+  if (usage_ == BufferUsage::HostVisible) {
+    for (size_t r = 0; r < rows; ++r) std::memcpy(static_cast<char *>(host_ptr) + r * width, static_cast<const char *>(ptr_) + r * pitch, width);
+    return true;
+  }
+  if (greta_cuda_memcpy_2d_d2h_sync(host_ptr, width, ptr_, pitch, width, rows) != GRETA_OK) return host::fail(err, host::cuda_error("D2H copy failed"));
+  return true;
+}
+
 GretaMemoryCuda::GretaMemoryCuda(size_t size, GretaDataType type, bool host_visible) {
   allocate(size, host_visible ? BufferUsage::HostVisible : BufferUsage::DeviceOnly, type, nullptr);
 }

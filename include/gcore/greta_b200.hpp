@@ -128,6 +128,8 @@ public:
   bool copy_to_device(const void *host_ptr, size_t size, std::string *err);
   bool copy_to_host(void *host_ptr, size_t size, std::string *err) const;
   bool copy_to_host_offset(void *host_ptr, size_t offset, size_t size, std::string *err) const;
+  // `rows` pieces of `width` bytes, `pitch` apart here, one behind the other in host memory.
+  bool copy_rows_to_host(void *host_ptr, size_t pitch, size_t width, size_t rows, std::string *err) const;
   bool copy_from_host(const void *src, size_t size) override { return copy_to_device(src, size, nullptr); }
   bool copy_to_host(void *dst, size_t size) const override { return copy_to_host(dst, size, nullptr); }
   void set_quant_info(const GretaQuantInfo &info) { qinfo_ = info; }

@@ -75,9 +75,27 @@ static int norm_out() {
   return 0;
 }
 
+// Buffer::copy_rows_to_host: rows apart on the device, together on the host; nothing beyond the buffer's end.
+static int copy_rows() {
+  gcore::rt::cuda::Buffer dev, pinned, none;
+  if (!dev.allocate(40, gcore::rt::cuda::BufferUsage::DeviceOnly, GretaDataType::INT8, &g_err) ||
+      !pinned.allocate(40, gcore::rt::cuda::BufferUsage::HostVisible, GretaDataType::INT8, &g_err))
+    return complain("allocate");
+  char src[40], got[40];
+  for (int i = 0; i < 40; ++i) src[i] = (char)i;
+  for (auto *b : {&dev, &pinned}) {
+    if (!b->copy_to_device(src, 40, &g_err) || !b->copy_rows_to_host(got, 14, 12, 3, &g_err)) return complain("copy_rows_to_host");
+    for (int r = 0; r < 3; ++r)
+      if (std::memcmp(got + 12 * r, src + 14 * r, 12) != 0) return complain("rows differ");
+    if (b->copy_rows_to_host(got, 14, 13, 3, nullptr) || b->copy_rows_to_host(got, 8, 8, 6, nullptr)) return complain("copied beyond the end");
+    if (!b->copy_rows_to_host(got, 14, 0, 3, &g_err) || !b->copy_rows_to_host(got, 14, 12, 0, &g_err)) return complain("an empty copy");
+  }
+  return none.copy_rows_to_host(got, 4, 4, 1, nullptr) ? complain("copied from a buffer that holds nothing") : 0;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
-  const int rc = what == "norm_out" ? norm_out() : 2;
+  const int rc = what == "norm_out" ? norm_out() : what == "copy_rows" ? copy_rows() : 2;
   printf("%s: %s\n", what.c_str(), rc ? "FAIL" : "PASS");
   return rc;
 }
