@@ -192,7 +192,7 @@ __global__ void embedding_kernel(const int32_t *tokens, const void *__restrict__
   }
 }
 
-// First maximum (lowest index among equal values) of each row of logits: a cluster of gridDim.x CTAs of 1024 threads per row
+// First maximum (lowest index among equal values; NaN counts only in the first place, where it wins) of each row of logits: a cluster of gridDim.x CTAs of 1024 threads per row
 // (per sequence of a batch).  One CTA per row is bound by the latency of its 32 dependent loads per thread, not by bandwidth: 15 us
 // of a 258 us step at 32000 logits; eight CTAs take 4 loads per thread, issued together, and meet through distributed shared memory.
 __global__ void __launch_bounds__(1024) argmax_kernel(const float *logits, uint32_t n,
@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *logits, uint3
 #pragma unroll 4
   for (uint32_t i = rank * blockDim.x + threadIdx.x; i < n; i += stride) {
     float v = logits[i];
+    if (v != v) v = i ? -INFINITY : INFINITY;  // as a scan from the first value on: a NaN is never greater, and nothing is greater than a NaN there
     if (v > best || bi == 0xffffffffu) {   // strided scan keeps the lowest index of this thread's maximum
       best = v;
       bi = i;

@@ -877,3 +877,28 @@ def test_rmsnorm_both(g, cols):
     g.check(lib.greta_cuda_rmsnorm_both(None, dx.ptr, dg.ptr, y2.ptr, h2.ptr, 3, cols, 1e-5))
     assert (y.download(np.uint32) == y2.download(np.uint32)).all()
     assert (h.download(np.uint16)[:3 * cols] == h2.download(np.uint16)[:3 * cols]).all()
+
+
+@pytest.mark.parametrize("n", [31, 4096, 8192, 16384, 32003, 128256])
+def test_argmax_of_rows_with_nan(g, n):
+    """The id is that of a scan from the first value on (a NaN is never greater, nothing is greater than a NaN in the first place), however many CTAs
+    share the row."""
+    rng = np.random.default_rng(n)
+    rows = rng.normal(0, 1, (6, n)).astype(np.float32)
+    rows[0, rng.choice(np.arange(1, n), size=n // 3, replace=False)] = np.nan
+    rows[1, 1:] = np.nan
+    rows[2, 0] = np.nan
+    rows[3] = np.nan
+    rows[4] = -np.inf
+    rows[4, n // 2:] = np.nan
+    rows[5, [n // 3, n - 1]] = np.nan, 50.0
+    out, lib = g.DeviceBuffer(6 * 4, zero=True), g.cuda()
+    g.check(lib.greta_cuda_argmax_advance_batch(None, _dev(g, rows).ptr, n, 6, out.ptr, None, None, None, 0))
+    want = []
+    for r in rows:
+        best = 0
+        for i in np.flatnonzero(~np.isnan(r)):
+            if r[i] > r[best]:
+                best = int(i)
+        want.append(best)
+    assert out.download(np.int32).tolist() == want and want[1:5] == [0, 0, 0, 0] and want[5] == n - 1
