@@ -2,6 +2,8 @@
 // decode path (norm, residual add, SwiGLU, embedding gather, greedy arg-max).
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "greta_common.cuh"
 
 using namespace greta;
@@ -163,32 +165,33 @@ __global__ void silu_mul_kernel(const float *g, const float *u, float *y, size_t
   }
 }
 
-// grid (rows, column groups of 256 * V); V = 4 where the row length and the pointers allow it.  One value per thread behind two 64-bit divisions
+// grid (rows, column groups of 256 * V, 65535 at most); V = 4 where the row length and the pointers allow it.  One value per thread behind two 64-bit divisions
 // took 10.5 us for 512 x 4096 and 28 for 1531.
 template <bool F16, int V>
 __global__ void embedding_kernel(const int32_t *tokens, const void *__restrict__ table, float *out, uint32_t dim, uint32_t vocab) {
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t s = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
-  if (c >= dim) return;
+  const uint32_t s = blockIdx.x;
   const int32_t t = tokens[s];
   const bool known = t >= 0 && t < (int32_t)vocab;
-  const size_t src = (size_t)(known ? t : 0) * dim + c;
-  float *o = out + (size_t)s * dim + c;
-  if (V == 4) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (known) {
-      if (F16) {
-        const uint2 u = *reinterpret_cast<const uint2 *>(reinterpret_cast<const __half *>(table) + src);
-        const float2 a = h2_to_f2(u.x), b = h2_to_f2(u.y);
-        v = make_float4(a.x, a.y, b.x, b.y);
-      } else {
-        v = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(table) + src);
+  for (size_t c = ((size_t)blockIdx.y * blockDim.x + threadIdx.x) * V; c < dim; c += (size_t)gridDim.y * blockDim.x * V) {
+    const size_t src = (size_t)(known ? t : 0) * dim + c;
+    float *o = out + (size_t)s * dim + c;
+    if (V == 4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (known) {
+        if (F16) {
+          const uint2 u = *reinterpret_cast<const uint2 *>(reinterpret_cast<const __half *>(table) + src);
+          const float2 a = h2_to_f2(u.x), b = h2_to_f2(u.y);
+          v = make_float4(a.x, a.y, b.x, b.y);
+        } else {
+          v = *reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(table) + src);
+        }
       }
+      *reinterpret_cast<float4 *>(o) = v;
+    } else {
+      *o = !known ? 0.f : F16 ? __half2float(reinterpret_cast<const __half *>(table)[src]) : reinterpret_cast<const float *>(table)[src];
     }
-    *reinterpret_cast<float4 *>(o) = v;
-  } else {
-    *o = !known ? 0.f : F16 ? __half2float(reinterpret_cast<const __half *>(table)[src]) : reinterpret_cast<const float *>(table)[src];
   }
 }
 
@@ -384,8 +387,7 @@ int greta_cuda_embedding(greta_stream_t stream, const int32_t *tokens, const voi
   if (n == 0) return GRETA_OK;
   GRETA_REQUIRE(tokens && table && out, "embedding: null pointer");
   const bool vec = dim % 4 == 0 && aligned16(out) && ((uintptr_t)table & (table_is_f16 ? 7u : 15u)) == 0;
-  const dim3 grid(Sq, (dim / (vec ? 4 : 1) + 255) / 256);
-  GRETA_REQUIRE(grid.y <= 65535, "embedding: dim=%u", dim);
+  const dim3 grid(Sq, std::min<size_t>(65535, ((size_t)dim / (vec ? 4 : 1) + 255) / 256));
   auto go = [&](auto kernel) { return launch_pdl(kernel, grid, dim3(256), 0, S(stream), tokens, table, out, dim, vocab); };
   GRETA_CUDA_TRY(table_is_f16 ? (vec ? go(embedding_kernel<true, 4>) : go(embedding_kernel<true, 1>))
                               : (vec ? go(embedding_kernel<false, 4>) : go(embedding_kernel<false, 1>)));

@@ -305,24 +305,25 @@ __global__ void embedding_positions_kernel(const int32_t *tokens, const void *__
                                            uint32_t vocab, uint32_t max_positions, const uint32_t *d_pos, uint32_t pos0) {
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t m = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * V, p = d_pos ? d_pos[m] : pos0 + m;
-  if (c >= D) return;
+  const uint32_t m = blockIdx.x, p = d_pos ? d_pos[m] : pos0 + m;
   const int32_t t = tokens[m];
   const bool known = t >= 0 && (uint32_t)t < vocab, placed = pos_table && p < max_positions;
-  float *o = out + (size_t)m * D + c;
-  if (V == 4) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (known) v = table_at4<T>(table, (size_t)t * D + c);
-    if (placed) {
-      const float4 w = table_at4<T>(pos_table, (size_t)p * D + c);
-      v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+  for (size_t c = ((size_t)blockIdx.y * blockDim.x + threadIdx.x) * V; c < D; c += (size_t)gridDim.y * blockDim.x * V) {
+    float *o = out + (size_t)m * D + c;
+    if (V == 4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (known) v = table_at4<T>(table, (size_t)t * D + c);
+      if (placed) {
+        const float4 w = table_at4<T>(pos_table, (size_t)p * D + c);
+        v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+      }
+      *reinterpret_cast<float4 *>(o) = v;
+    } else {
+      float v = 0.f;
+      if (known) v = table_at<T>(table, (size_t)t * D + c);
+      if (placed) v += table_at<T>(pos_table, (size_t)p * D + c);
+      *o = v;
     }
-    *reinterpret_cast<float4 *>(o) = v;
-  } else {
-    float v = 0.f;
-    if (known) v = table_at<T>(table, (size_t)t * D + c);
-    if (placed) v += table_at<T>(pos_table, (size_t)p * D + c);
-    *o = v;
   }
 }
 
@@ -330,20 +331,21 @@ template <typename T, int V>
 __global__ void embedding_scaled_kernel(const int32_t *tokens, const T *__restrict__ table, uint32_t ld, float scale, float *out, uint32_t D, uint32_t vocab) {
   pdl_launch_dependents();
   pdl_wait();
-  const uint32_t m = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
-  if (c >= D) return;
+  const uint32_t m = blockIdx.x;
   const int32_t t = tokens[m];
   const bool known = t >= 0 && (uint32_t)t < vocab;
-  float *o = out + (size_t)m * D + c;
-  if (V == 4) {
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (known) {
-      v = table_at4<T>(table, (size_t)t * ld + c);
-      v = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+  for (size_t c = ((size_t)blockIdx.y * blockDim.x + threadIdx.x) * V; c < D; c += (size_t)gridDim.y * blockDim.x * V) {
+    float *o = out + (size_t)m * D + c;
+    if (V == 4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (known) {
+        v = table_at4<T>(table, (size_t)t * ld + c);
+        v = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+      }
+      *reinterpret_cast<float4 *>(o) = v;
+    } else {
+      *o = known ? table_at<T>(table, (size_t)t * ld + c) * scale : 0.f;
     }
-    *reinterpret_cast<float4 *>(o) = v;
-  } else {
-    *o = known ? table_at<T>(table, (size_t)t * ld + c) * scale : 0.f;
   }
 }
 
@@ -453,8 +455,7 @@ int greta_cuda_embedding_positions(greta_stream_t stream, const int32_t *tokens,
   GRETA_REQUIRE(tokens && table && out, "embedding_positions: null pointer");
   GRETA_REQUIRE(fmt == GRETA_FMT_BF16 || fmt == GRETA_FMT_F32, "embedding_positions: table format %d", fmt);
   const bool vec = D % 4 == 0 && aligned16(out) && (((uintptr_t)table | (uintptr_t)pos_table) & (fmt == GRETA_FMT_BF16 ? 7u : 15u)) == 0;
-  const dim3 grid(M, (D / (vec ? 4 : 1) + 255) / 256);
-  GRETA_REQUIRE(grid.y <= 65535, "embedding_positions: width %u", D);
+  const dim3 grid(M, std::min<size_t>(65535, ((size_t)D / (vec ? 4 : 1) + 255) / 256));
   auto go = [&](auto kernel) {
     return launch_pdl(kernel, grid, dim3(256), 0, (cudaStream_t)stream, tokens, table, pos_table, out, D, vocab, max_positions, d_pos, pos0);
   };
@@ -469,8 +470,7 @@ int greta_cuda_embedding_scaled(greta_stream_t stream, const int32_t *tokens, co
   GRETA_REQUIRE(tokens && table && out && ld >= D, "embedding_scaled: bad argument");
   GRETA_REQUIRE(fmt == GRETA_FMT_BF16 || fmt == GRETA_FMT_F32, "embedding_scaled: table format %d", fmt);
   const bool vec = D % 4 == 0 && ld % 4 == 0 && aligned16(out) && ((uintptr_t)table & (fmt == GRETA_FMT_BF16 ? 7u : 15u)) == 0;
-  const dim3 grid(M, (D / (vec ? 4 : 1) + 255) / 256);
-  GRETA_REQUIRE(grid.y <= 65535, "embedding_scaled: width %u", D);
+  const dim3 grid(M, std::min<size_t>(65535, ((size_t)D / (vec ? 4 : 1) + 255) / 256));
   auto go = [&](auto kernel, auto *rows) { return launch_pdl(kernel, grid, dim3(256), 0, (cudaStream_t)stream, tokens, rows, ld, scale, out, D, vocab); };
   const __nv_bfloat16 *t16 = static_cast<const __nv_bfloat16 *>(table);
   const float *t32 = static_cast<const float *>(table);

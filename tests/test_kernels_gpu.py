@@ -902,3 +902,20 @@ def test_argmax_of_rows_with_nan(g, n):
                 best = int(i)
         want.append(best)
     assert out.download(np.int32).tolist() == want and want[1:5] == [0, 0, 0, 0] and want[5] == n - 1
+
+
+@pytest.mark.parametrize("op", ["embedding", "embedding_positions", "embedding_scaled"])
+def test_embedding_rows_wider_than_the_grid(g, op):
+    """A row of odd length beyond 65535 groups of 256 columns."""
+    D, lib = 65535 * 256 + 3, g.cuda()
+    table = np.random.default_rng(1).normal(0, 1, (2, D)).astype(np.float32)
+    tok, t, out = _dev(g, np.array([1, 7], np.int32)), _dev(g, table), g.DeviceBuffer(2 * D * 4)
+    _KEEP.append(out)
+    if op == "embedding":
+        g.check(lib.greta_cuda_embedding(None, tok.ptr, t.ptr, 0, out.ptr, 2, D, 2))
+    elif op == "embedding_positions":
+        g.check(lib.greta_cuda_embedding_positions(None, tok.ptr, t.ptr, None, g.FMT_F32, out.ptr, 2, D, 2, 0, None, 0))
+    else:
+        g.check(lib.greta_cuda_embedding_scaled(None, tok.ptr, t.ptr, g.FMT_F32, D, 1.0, out.ptr, 2, D, 2))
+    got = out.download(np.float32).reshape(2, D)
+    assert (got[0] == table[1]).all() and (got[1] == 0).all()   # an id beyond the vocabulary gives zeros
