@@ -367,6 +367,24 @@ uint32_t pick_tokens(uint32_t M, uint32_t row_tiles, uint32_t KT, uint32_t sms) 
   return best;
 }
 
+// Row tiles of `rows` weight rows, and the launch that they and M tokens make.
+uint32_t row_tiles_of(uint32_t rows, int mode) {
+  const uint32_t tile_rows = mode == GRETA_GEMM_SWIGLU_F16 ? TILE_N / 2 : TILE_N;
+  return (rows + tile_rows - 1) / tile_rows;
+}
+struct TsPlan {
+  uint32_t tn, accs, w_slots, act_stages, tok_tiles;
+};
+TsPlan plan_ts(uint32_t M, uint32_t K, uint32_t row_tiles) {
+  TsPlan p;
+  p.tn = pick_tokens(M, row_tiles, (K + 2 * TS_K - 1) / (2 * TS_K) * 2, (uint32_t)sm_count());
+  p.accs = p.tn <= 192 ? 2 : 1;  // two accumulators and at least two weight slots
+  p.w_slots = TS_TMEM - p.accs * p.tn >= 4 * TS_W_COLS ? 4 : 2;
+  p.act_stages = stages_of(p.tn);
+  p.tok_tiles = (M + p.tn - 1) / p.tn;
+  return p;
+}
+
 template <int FMT, int MODE>
 int launch_ts(cudaStream_t stream, const TsArgs &a, uint32_t sms, size_t smem) {
   static bool attr_set[64] = {};
@@ -399,6 +417,20 @@ extern "C" int greta_cuda_gemm_segments_status(greta_stream_t stream, int *code)
   return GRETA_OK;
 }
 
+extern "C" int greta_cuda_gemm_segments_route(uint32_t M, uint32_t K, const uint32_t *n, uint32_t n_segs, int mode, uint32_t *tile_tokens,
+                                              uint32_t *accumulators, uint32_t *weight_slots, uint32_t *tiles) {
+  GRETA_REQUIRE(n && n_segs >= 1 && n_segs <= 3 && tile_tokens && accumulators && weight_slots && tiles, "gemm_segments_route: bad argument");
+  GRETA_REQUIRE(M && K && K % 32 == 0 && mode >= GRETA_GEMM_STORE && mode <= GRETA_GEMM_SWIGLU_F16, "gemm_segments_route: M=%u K=%u mode %d", M, K, mode);
+  uint32_t row_tiles = 0;
+  for (uint32_t i = 0; i < (mode == GRETA_GEMM_SWIGLU_F16 ? 1 : n_segs); ++i) row_tiles += row_tiles_of(n[i], mode);
+  const TsPlan p = plan_ts(M, K, row_tiles);
+  *tile_tokens = p.tn;
+  *accumulators = p.accs;
+  *weight_slots = p.w_slots;
+  *tiles = row_tiles * p.tok_tiles;
+  return GRETA_OK;
+}
+
 extern "C" int greta_cuda_gemm_segments(greta_stream_t stream, int fmt, const void *a_f16, uint32_t M, uint32_t K, const greta_gemm_segment *segs,
                                         uint32_t n_segs, int mode) {
   GRETA_REQUIRE(fmt == GRETA_FMT_Q4_0 || fmt == GRETA_FMT_Q8_0, "gemm_segments: format %d is not supported (Q4_0 or Q8_0)", fmt);
@@ -424,7 +456,7 @@ extern "C" int greta_cuda_gemm_segments(greta_stream_t stream, int fmt, const vo
     GRETA_REQUIRE(aligned16(g.qs) && aligned16(g.d) && ((uintptr_t)g.out & 3) == 0, "gemm_segments: segment %u is misaligned", i);
     w.out[i] = static_cast<float *>(g.out);
     w.n[i] = g.n;
-    if (!pair || i == 0) row_tiles += (g.n + tile_rows - 1) / tile_rows;
+    if (!pair || i == 0) row_tiles += row_tiles_of(g.n, mode);
     w.tile_end[i] = row_tiles;
     const cuuint64_t qd[2] = {row_bytes, g.n}, qs[1] = {row_bytes}, dd[2] = {nb, g.n}, ds[1] = {(cuuint64_t)d_row_stride(nb) * 2};
     const cuuint32_t qbox[2] = {128, tile_rows}, dbox[2] = {8, tile_rows}, one[2] = {1, 1};
@@ -439,16 +471,17 @@ extern "C" int greta_cuda_gemm_segments(greta_stream_t stream, int fmt, const vo
     }
   }
   for (uint32_t i = n_segs; i < 3; ++i) w.tile_end[i] = row_tiles;
-  const uint32_t tn = pick_tokens(M, row_tiles, KT, sms);
+  const TsPlan plan = plan_ts(M, K, row_tiles);
+  const uint32_t tn = plan.tn;
   w.M = M;
   w.K = K;
   w.tn = tn;
-  w.tok_tiles = (M + tn - 1) / tn;
+  w.tok_tiles = plan.tok_tiles;
   GRETA_REQUIRE((uint64_t)row_tiles * w.tok_tiles * KT < (1ull << 31), "gemm_segments: M=%u K=%u: too many tiles", M, K);
   w.tiles = row_tiles * w.tok_tiles;
-  w.act_stages = stages_of(tn);
-  w.accs = tn <= 192 ? 2 : 1;  // two accumulators and at least two weight slots
-  w.w_slots = TS_TMEM - w.accs * tn >= 4 * TS_W_COLS ? 4 : 2;
+  w.act_stages = plan.act_stages;
+  w.accs = plan.accs;
+  w.w_slots = plan.w_slots;
   w.idesc = instr_desc_f16(TILE_N, tn);
   const cuuint64_t ad[2] = {K, M}, as[1] = {(cuuint64_t)K * 2};
   const cuuint32_t abox[2] = {BK, tn}, one[2] = {1, 1};

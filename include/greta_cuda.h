@@ -328,6 +328,10 @@ typedef struct greta_gemm_segment {
 } greta_gemm_segment;
 GRETA_API int greta_cuda_gemm_segments(greta_stream_t stream, int fmt, const void *a_f16, uint32_t M, uint32_t K, const greta_gemm_segment *segs,
                                        uint32_t n_segs, int mode);
+/* How it would cut that product, n[i] rows per segment (nothing is launched): tokens per tile, accumulators and weight operands held in tensor
+ * memory, tiles of the launch (one persistent CTA per SM goes through them). */
+GRETA_API int greta_cuda_gemm_segments_route(uint32_t M, uint32_t K, const uint32_t *n, uint32_t n_segs, int mode, uint32_t *tile_tokens,
+                                             uint32_t *accumulators, uint32_t *weight_slots, uint32_t *tiles);
 /* The code of its kernels so far on the stream: valid in *code once the stream has been synchronised (*code in page-locked memory). */
 GRETA_API int greta_cuda_gemm_segments_status(greta_stream_t stream, int *code);
 

@@ -1,13 +1,19 @@
 // Drives BlockScheduler from C++ where the C interface does not reach: buffers that it exposes and the tensor-parallel hooks.  The first
 // argument names the check; exits non-zero when it fails.  Built by gretacore-v3_b200/csrc/Makefile (target scheduler_test) and run by
 // tests/test_scheduler_gpu.py.
+#include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "gcore/inference/block_scheduler.hpp"
+#include "greta_cuda.h"
 
 using namespace gcore::inference;
 using gcore::rt::GretaDataType;
@@ -93,9 +99,91 @@ static int copy_rows() {
   return none.copy_rows_to_host(got, 4, 4, 1, nullptr) ? complain("copied from a buffer that holds nothing") : 0;
 }
 
+// The prompt of a tensor-parallel model, two ranks as two threads on one GPU: the all-reduce hook waits for its own stream, and the ranks meet
+// on the host (no kernel waits for another rank's).  Hidden rows and logits against the same model on one rank, on either side of 32 rows and
+// behind an earlier portion.
+struct Meeting {
+  std::mutex m;
+  std::condition_variable cv;
+  std::vector<float> sum;
+  int arrived = 0, round = 0;
+  void add(std::vector<float> &v) {
+    std::unique_lock<std::mutex> lock(m);
+    if (arrived == 0) sum.assign(v.size(), 0.0f);
+    for (size_t i = 0; i < v.size(); ++i) sum[i] += v[i];
+    const int now = round;
+    if (++arrived == 2) {
+      arrived = 0;
+      ++round;
+      cv.notify_all();
+    } else if (!cv.wait_for(lock, std::chrono::seconds(60), [&] { return round != now; })) {
+      std::fprintf(stderr, "the other rank did not come\n");
+      std::exit(1);
+    }
+    v = sum;
+  }
+};
+static int tensor_parallel() {
+  const ModelConfig c = small();
+  const std::vector<int32_t> t = prompt(150);
+  const size_t parts[] = {20, 40, 90};
+  struct Result {
+    std::vector<std::vector<float>> hidden, logits;
+    std::string err;
+    bool ok = false;
+  } one, two[2];
+  Meeting meet;
+  auto run = [&](ModelConfig k, Result *out) {
+    BlockScheduler s;
+    if (!(s.init(k, &out->err) && s.allocate_weights(&out->err) && s.load_synthetic_weights(5, &out->err) && s.allocate_activations(1, k.max_seq_len, &out->err))) return;
+    if (k.tp_size > 1)
+      s.set_all_reduce([&](float *buf, size_t count, cudaStream_t stream) {
+        std::vector<float> v(count);
+        if (greta_cuda_stream_synchronize((greta_stream_t)stream) != GRETA_OK || greta_cuda_memcpy_d2h_sync(v.data(), buf, count * 4) != GRETA_OK) return 1;
+        meet.add(v);
+        return greta_cuda_memcpy_h2d_sync(buf, v.data(), count * 4) == GRETA_OK ? 0 : 1;
+      });
+    size_t pos = 0;
+    for (size_t n : parts) {
+      if (!s.forward(t.data() + pos, pos, n, &out->err)) return;
+      pos += n;
+      std::vector<float> h(n * k.dim), z(k.vocab_size);
+      if (!s.get_hidden_state().copy_to_host(h.data(), h.size() * 4, &out->err) || !s.get_logits().copy_to_host(z.data(), z.size() * 4, &out->err)) return;
+      out->hidden.push_back(std::move(h));
+      out->logits.push_back(std::move(z));
+    }
+    out->ok = true;
+  };
+  run(c, &one);
+  std::vector<std::thread> ranks;
+  for (uint32_t r = 0; r < 2; ++r) {
+    ModelConfig k = c;
+    k.tp_size = 2;
+    k.tp_rank = r;
+    ranks.emplace_back(run, k, &two[r]);
+  }
+  for (auto &th : ranks) th.join();
+  for (const Result *r : {&one, &two[0], &two[1]})
+    if (!r->ok) return fprintf(stderr, "%s\n", r->err.c_str()), 1;
+  for (size_t p = 0; p < 3; ++p)
+    for (const Result &r : two) {
+      const std::vector<float> *pairs[2][2] = {{&one.hidden[p], &r.hidden[p]}, {&one.logits[p], &r.logits[p]}};
+      for (auto &ab : pairs) {
+        double worst = 0, top = 0;
+        for (size_t i = 0; i < ab[0]->size(); ++i) {
+          worst = std::fmax(worst, std::fabs((double)(*ab[0])[i] - (*ab[1])[i]));
+          top = std::fmax(top, std::fabs((double)(*ab[0])[i]));
+        }
+        // fp32 sums in another order; above 32 rows a value may round to the next fp16 (2^-11) on the way into a product
+        if (!(worst <= (parts[p] > 32 || p ? 1e-3 : 1e-5) * top)) return fprintf(stderr, "portion %zu: %g of %g\n", p, worst, top), 1;
+      }
+    }
+  return 0;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
-  const int rc = what == "norm_out" ? norm_out() : what == "copy_rows" ? copy_rows() : 2;
+  const int rc = what == "norm_out" ? norm_out() : what == "copy_rows" ? copy_rows() : what == "tensor_parallel" ? tensor_parallel() : 2;
   printf("%s: %s\n", what.c_str(), rc ? "FAIL" : "PASS");
   return rc;
 }

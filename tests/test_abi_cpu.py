@@ -105,3 +105,21 @@ def test_gemm_route_arithmetic():
         assert route(512, 384, 4096, 1)[0] == 0                            # too few tiles for 512-token tiles: not paired
     finally:
         assert lib.greta_cuda_set_tuning(b"gemm_pair", 0) == 0
+
+
+def test_gemm_segments_route_is_host_arithmetic(pkg):
+    lib = pkg.ffi.cuda()
+    out = [C.c_uint32() for _ in range(4)]
+    ptr = [C.addressof(v) for v in out]
+    n = (C.c_uint32 * 3)(4096, 1024, 1024)
+    np_ = C.cast(n, C.c_void_p)
+
+    def route(M, K, n_segs, mode):
+        return lib.greta_cuda_gemm_segments_route(M, K, np_, n_segs, mode, *ptr)
+
+    assert route(1531, 4096, 3, 0) == 0
+    tokens, accs, slots, tiles = (v.value for v in out)
+    assert tokens % 32 == 0 and 32 <= tokens <= 256 and accs * tokens + slots * 64 <= 512 and tiles == (32 + 8 + 8) * -(-1531 // tokens)
+    assert route(40, 4096, 2, 2) == 0 and out[3].value == 64 * -(-40 // out[0].value)   # gate and up: tiles of 64 rows of either
+    assert route(40, 48, 1, 0) == 4 and route(0, 64, 1, 0) == 4 and route(40, 64, 4, 0) == 4 and route(40, 64, 1, 3) == 4
+    assert lib.greta_cuda_gemm_segments_route(40, 64, None, 1, 0, *ptr) == 4

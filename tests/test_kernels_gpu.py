@@ -919,3 +919,58 @@ def test_embedding_rows_wider_than_the_grid(g, op):
         g.check(lib.greta_cuda_embedding_scaled(None, tok.ptr, t.ptr, g.FMT_F32, D, 1.0, out.ptr, 2, D, 2))
     got = out.download(np.float32).reshape(2, D)
     assert (got[0] == table[1]).all() and (got[1] == 0).all()   # an id beyond the vocabulary gives zeros
+
+
+# (mode, tokens, K, rows per segment, tokens per tile, accumulators, weight operands, more tiles than this many per CTA) on 148 SMs
+SEGMENT_FORMS = [
+    (0, 129, 256, (8192,), 96, 2, 4, 0), (0, 97, 256, (4096,) * 3, 128, 2, 4, 0), (0, 1000, 256, (8192,), 128, 2, 4, 3), (0, 257, 256, (8192,), 160, 2, 2, 0),
+    (0, 2047, 256, (4096,), 160, 2, 2, 2), (0, 1000, 256, (4096,) * 3, 192, 2, 2, 3), (0, 200, 2048, (4096,) * 3, 224, 1, 4, 0),
+    (0, 2047, 4096, (2048,), 256, 1, 4, 0),
+    (1, 129, 256, (8192,), 96, 2, 4, 0), (1, 1000, 256, (8192,), 128, 2, 4, 3), (1, 2047, 256, (4096,), 160, 2, 2, 2), (1, 3001, 256, (4096,), 192, 2, 2, 3),
+    (1, 200, 2048, (11008,), 224, 1, 4, 0), (1, 2047, 4096, (2048,), 256, 1, 4, 0), (1, 1024, 28672, (8192,), 256, 1, 4, 1),
+    (2, 257, 256, (8192,), 96, 2, 4, 2), (2, 1000, 256, (4096,), 128, 2, 4, 3), (2, 450, 256, (8192,), 160, 2, 2, 2), (2, 700, 256, (8192,), 192, 2, 2, 3),
+    (2, 200, 1024, (8192,), 224, 1, 4, 0), (2, 2047, 4096, (1000,), 256, 1, 4, 0)]
+
+
+@pytest.mark.parametrize("name", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("mode,M,K,ns,tokens,accs,slots,per_cta", SEGMENT_FORMS)
+def test_gemm_segments_forms(g, name, mode, M, K, ns, tokens, accs, slots, per_cta):
+    """Every tile width, one and two accumulators, two and four weight operands, for each epilogue, with a single tile per CTA and with several (accumulators,
+    barriers and the gate / up exchange used again).  The results are the bits of the operators that the launch replaces."""
+    if K > 8192 and name == "q8_0":
+        pytest.skip("one format is enough for the largest product")
+    lib = g.cuda()
+    got = [C.c_uint32() for _ in range(4)]
+    rows = (C.c_uint32 * 2)(*ns) if len(ns) < 3 else (C.c_uint32 * 3)(*ns)
+    g.check(lib.greta_cuda_gemm_segments_route(M, K, C.cast(rows, C.c_void_p), len(ns), mode, *[C.addressof(v) for v in got]))
+    assert [v.value for v in got[:3]] == [tokens, accs, slots] and got[3].value > per_cta * 148
+    ofmt, gfmt = FMTS[name]
+    rng = np.random.default_rng(M + K + mode)
+    a16 = rng.standard_normal((M, K), dtype=np.float32).astype(np.float16).view(np.uint16)
+    ns = ns * 2 if mode == 2 else ns
+    w = [g.Weight(make_blocks(rng, ofmt, n, K), gfmt, n, K) for n in ns]
+    base = [rng.standard_normal((M + 1, n), dtype=np.float32) for n in ns]
+    a, outs = _dev(g, a16), [_dev(g, b) for b in base]
+    segs = (_Segment * len(ns))(*[_Segment(x.qs.ptr, x.d.ptr, n, o.ptr) for x, n, o in zip(w, ns, outs)])
+    g.check(lib.greta_cuda_gemm_segments(None, gfmt, a.ptr, M, K, C.cast(segs, C.c_void_p), len(ns), mode))
+    g.check(lib.greta_cuda_device_synchronize())
+    assert _gemm_status(g) == 0
+    single = []
+    for x, n in zip(w, ns):
+        c = g.DeviceBuffer(M * n * 4)
+        _KEEP.append(c)
+        g.check(lib.greta_cuda_gemm(None, gfmt, a.ptr, 1, x.qs.ptr, x.d.ptr, c.ptr, 0, M, n, K, None))
+        single.append(c)
+    if mode == 2:
+        h = g.DeviceBuffer(M * ns[0] * 2)
+        _KEEP.append(h)
+        g.check(lib.greta_cuda_silu_mul(None, single[0].ptr, single[1].ptr, single[0].ptr, M * ns[0]))
+        g.check(lib.greta_cuda_f32_to_f16(None, single[0].ptr, h.ptr, M * ns[0]))
+        out = outs[0].download(np.uint16)
+        assert (out[:M * ns[0]] == h.download(np.uint16)).all()
+        assert (out[M * ns[0]:] == base[0].view(np.uint16).reshape(-1)[M * ns[0]:]).all()
+        return
+    for o, b, s in zip(outs, base, single):
+        out, s = o.download(np.float32).reshape(b.shape), s.download(np.float32).reshape(M, -1)
+        assert (out[M] == b[M]).all()
+        assert (out[:M] == (b[:M] + s if mode == 1 else s)).all()
