@@ -110,18 +110,17 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ 
 
 // The same values as fp16, for the tensor-core products.  A row stays in registers (PER values per thread, all loads under way together;
 // the 256-thread order of the sum is rmsnorm_kernel's, so the results are its bits): 3.8 us for 512 x 4096 in the layer against 10.8 and a
-// conversion pass of 2.9 per product.  y32 may be null; otherwise it takes the fp32 values as well.
-template <int PER>
+// conversion pass of 2.9 per product.  BOTH: y32 takes the fp32 values as well.
+template <int PER, bool BOTH>
 __global__ void __launch_bounds__(256) rmsnorm_f16_kernel(const float *x, const float *__restrict__ gamma, __half *y, float *y32, uint32_t cols, float eps) {
   __shared__ float sm[32];
   pdl_launch_dependents();
   pdl_wait();
   const float *xr = x + (size_t)blockIdx.x * cols;
   __half *yr = y + (size_t)blockIdx.x * cols;
-  float *y32r = y32 ? y32 + (size_t)blockIdx.x * cols : nullptr;
   auto put = [&](uint32_t c, float n) {
     yr[c] = __float2half_rn(n);
-    if (y32r) y32r[c] = n;
+    if (BOTH) y32[(size_t)blockIdx.x * cols + c] = n;
   };
   float v[PER], ss = 0.f;
 #pragma unroll
@@ -174,7 +173,7 @@ __global__ void embedding_kernel(const int32_t *tokens, const void *__restrict__
   const uint32_t s = blockIdx.x;
   const int32_t t = tokens[s];
   const bool known = t >= 0 && t < (int32_t)vocab;
-  for (size_t c = ((size_t)blockIdx.y * blockDim.x + threadIdx.x) * V; c < dim; c += (size_t)gridDim.y * blockDim.x * V) {
+  for (uint32_t c = first_column<V>(); c < dim; c = next_column<V>(c, dim)) {
     const size_t src = (size_t)(known ? t : 0) * dim + c;
     float *o = out + (size_t)s * dim + c;
     if (V == 4) {
@@ -288,7 +287,12 @@ int launch_argmax(cudaStream_t stream, const float *logits, uint32_t n, uint32_t
 
 int launch_rmsnorm_f16(cudaStream_t stream, const float *x, const float *gamma, void *y, float *y32, uint32_t rows, uint32_t cols, float eps) {
   auto go = [&](auto kernel) { return launch_pdl(kernel, dim3(rows), dim3(256), 0, stream, x, gamma, static_cast<__half *>(y), y32, cols, eps); };
-  GRETA_CUDA_TRY(cols <= 256 * 8 ? go(rmsnorm_f16_kernel<8>) : cols <= 256 * 16 ? go(rmsnorm_f16_kernel<16>) : go(rmsnorm_f16_kernel<32>));
+  if (cols <= 256 * 8)
+    GRETA_CUDA_TRY(y32 ? go(rmsnorm_f16_kernel<8, true>) : go(rmsnorm_f16_kernel<8, false>));
+  else if (cols <= 256 * 16)
+    GRETA_CUDA_TRY(y32 ? go(rmsnorm_f16_kernel<16, true>) : go(rmsnorm_f16_kernel<16, false>));
+  else
+    GRETA_CUDA_TRY(y32 ? go(rmsnorm_f16_kernel<32, true>) : go(rmsnorm_f16_kernel<32, false>));
   return launched("rmsnorm_f16_kernel");
 }
 

@@ -308,7 +308,7 @@ __global__ void embedding_positions_kernel(const int32_t *tokens, const void *__
   const uint32_t m = blockIdx.x, p = d_pos ? d_pos[m] : pos0 + m;
   const int32_t t = tokens[m];
   const bool known = t >= 0 && (uint32_t)t < vocab, placed = pos_table && p < max_positions;
-  for (size_t c = ((size_t)blockIdx.y * blockDim.x + threadIdx.x) * V; c < D; c += (size_t)gridDim.y * blockDim.x * V) {
+  for (uint32_t c = first_column<V>(); c < D; c = next_column<V>(c, D)) {
     float *o = out + (size_t)m * D + c;
     if (V == 4) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -334,7 +334,7 @@ __global__ void embedding_scaled_kernel(const int32_t *tokens, const T *__restri
   const uint32_t m = blockIdx.x;
   const int32_t t = tokens[m];
   const bool known = t >= 0 && (uint32_t)t < vocab;
-  for (size_t c = ((size_t)blockIdx.y * blockDim.x + threadIdx.x) * V; c < D; c += (size_t)gridDim.y * blockDim.x * V) {
+  for (uint32_t c = first_column<V>(); c < D; c = next_column<V>(c, D)) {
     float *o = out + (size_t)m * D + c;
     if (V == 4) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
