@@ -19,10 +19,10 @@
 // A gate / up tile is 64 rows of either matrix: its accumulator has gate in lanes 0-63 and up in lanes 64-127 and the two meet through shared
 // memory, so the tile costs what any other does (a tile of 128 rows of both needs two accumulators, which leaves half the weight slots: 115
 // against 91 us at 512 tokens x 4096 x 2 x 11008).
-// Measured alone with a cold L2 (launch and event overhead included), 512 tokens, Q4_0: 3 x 4096 x 4096 52 us = 995 TFLOP/s, 4096 x 4096
-// 32 us, 4096 x 11008 56 us; gemm_tc.cu in the model: 138, 46 and 93 us.  1531 tokens, 2 x 14336 x 4096: 270 us = 1330 TFLOP/s (0.83 of the
-// measured peak), gemm_tc.cu 358 us and a SwiGLU pass of 108.  What is left: the last tile's end (25 ns per token column) and waves that
-// do not fill the SMs.
+// Measured alone with a cold L2 (median, launch and event overhead included; greta_cuda_gemm's kernel timed the same way behind the stroke), 512
+// tokens, Q4_0: 3 x 4096 x 4096 52 / 120 us = 990 TFLOP/s, 4096 x 4096 29 / 43, 4096 x 11008 53 / 88, 2 x 11008 x 4096 with SwiGLU 92 / 114 without.
+// 1531 tokens, Q8_0: 2 x 14336 x 4096 280 / 362 us = 1282 TFLOP/s (0.77 of the measured peak), 4096 x 14336 148 / 184.  What is left: the last
+// tile's end (25 ns per token column) and waves that do not fill the SMs.
 // Every wait is bounded: on a timeout the kernel raises a flag that all roles poll, drains, frees its tensor memory and returns;
 // greta_cuda_gemm_status() reports it.
 #include "gemm_dequant.cuh"

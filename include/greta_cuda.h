@@ -128,7 +128,8 @@ GRETA_API int greta_cuda_set_pdl(int on);
  *   0 = automatic), "gemm_splitk" (GRETA_GEMM_SPLITK, default 0: 1 = a prefill GEMM with fewer 512-token tiles than
  *   SMs shares each tile's K loop between CTAs where that is predicted to pay, 2 = wherever it is feasible; needs the workspace; the partial sums change the
  *   fp32 summation order, deterministically), "gemm_pair" (GRETA_GEMM_PAIR: 1 = prefill GEMMs that take 512-token tiles
- *   run as pairs of CTAs sharing one two-CTA tensor-core instruction, 2 = every GEMM does, 0 = none). */
+ *   run as pairs of CTAs sharing one two-CTA tensor-core instruction, 2 = every GEMM does, 0 = none).
+ * The three "gemm_" switches act on greta_cuda_gemm; a model's prompt goes through greta_cuda_gemm_segments, which has none. */
 GRETA_API int greta_cuda_set_tuning(const char *name, long long value);
 /* Number of kernel launches this library has issued on the calling process (all threads). */
 GRETA_API uint64_t greta_cuda_launch_count(void);
