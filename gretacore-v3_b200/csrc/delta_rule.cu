@@ -23,6 +23,7 @@
 // short convolution first (gated_prepare_kernel; in decode inside gated_step_kernel).
 #include <algorithm>
 
+#include "delta_scan.cuh"
 #include "dense_device.cuh"
 
 using namespace greta;
@@ -30,7 +31,6 @@ using namespace greta;
 namespace {
 
 constexpr uint32_t DR_LANES = 8;
-__host__ __device__ constexpr uint32_t dim32(uint32_t d) { return (d + 31u) & ~31u; }
 
 __device__ __forceinline__ float sum8(float v) {  // over the eight lanes of a column
   v += __shfl_xor_sync(0xffffffffu, v, 1);
@@ -124,22 +124,6 @@ __global__ void __launch_bounds__(512) delta_step_kernel(const __grid_constant__
   for (uint32_t i = threadIdx.x; i < D; i += blockDim.x)
     store_out(out, out_fmt, (size_t)m * ld_out + (size_t)h * D + i, so[i] * inv * d.norm[(size_t)h * D + i] * d.gate[at + i]);
 }
-
-__device__ __forceinline__ void cp16(void *dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp4(void *dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-
-// What the scan reads, for either form: rows of consecutive tokens.
-struct ScanArgs {
-  const float *w, *k, *a, *r, *v;  // decay, key, removal rate (general) or write strength per head (gated), receptance / query, value
-  uint32_t ld_w, ld_k, ld_a, ld_r, ld_v;
-  uint32_t heads, per, dim, vdim;  // per: value heads that share a query / key head
-  uint32_t T, pos0, slot;
-  float *state;
-};
 
 // The recurrence over a portion: grid (heads, column groups).  A CTA keeps COLS columns of one head in the registers of its
 // first warps, NC columns per group of eight lanes, and walks the tokens in chunks of TC = a block per producer warp.
@@ -755,8 +739,7 @@ int launch_scan(cudaStream_t s, const ScanArgs &a, float *o_buf, int vec) {
 }
 template <bool GATED>
 int pick_scan(cudaStream_t s, const ScanArgs &a, float *o_buf) {
-  const int vec = a.dim % 4 == 0 && a.vdim % 4 == 0 && a.ld_w % 4 == 0 && a.ld_k % 4 == 0 && a.ld_r % 4 == 0 && a.ld_v % 4 == 0 && aligned16(a.w) &&
-                  aligned16(a.k) && aligned16(a.r) && aligned16(a.v) && (GATED || (a.ld_a % 4 == 0 && aligned16(a.a)));
+  const int vec = scan_vec(a, GATED);
   // Few heads: half the columns per CTA where the doubled grid still has an SM for every CTA (the usual head sizes).
   const bool narrow = a.heads * ((a.vdim + 15) / 16) <= (uint32_t)sm_count();
   switch (dim32(a.dim) / 32) {
@@ -769,6 +752,12 @@ int pick_scan(cudaStream_t s, const ScanArgs &a, float *o_buf) {
     case 7: return launch_scan<7, 1, 32, GATED>(s, a, o_buf, vec);
     default: return launch_scan<8, 1, 32, GATED>(s, a, o_buf, vec);
   }
+}
+// Portions take the chunked form where it covers them.
+template <bool GATED>
+int scan(cudaStream_t s, const ScanArgs &a, float *o_buf, void *scratch, size_t scratch_bytes) {
+  const size_t need = chunk_scan_bytes(a.heads, a.dim, a.vdim, GATED, a.T);
+  return need && scratch && aligned16(scratch) && scratch_bytes >= need ? chunk_scan(s, a, GATED, o_buf, static_cast<float *>(scratch)) : pick_scan<GATED>(s, a, o_buf);
 }
 int launch_output(cudaStream_t s, const OutArgs &a, const float *o_buf, void *out, int out_fmt, uint32_t ld_out) {
   const uint32_t D = a.dim, pairs = a.M * a.heads;
@@ -816,11 +805,15 @@ int greta_cuda_delta_step(greta_stream_t stream, const greta_delta_rule *d, cons
 }
 
 int greta_cuda_delta_scan(greta_stream_t stream, const greta_delta_rule *d, const greta_rows *rows, float *o_buf) {
+  return greta_cuda_delta_scan_chunked(stream, d, rows, o_buf, nullptr, 0);
+}
+size_t greta_cuda_delta_scan_scratch_bytes(uint32_t heads, uint32_t dim, uint32_t rows) { return chunk_scan_bytes(heads, dim, dim, false, rows); }
+int greta_cuda_delta_scan_chunked(greta_stream_t stream, const greta_delta_rule *d, const greta_rows *rows, float *o_buf, void *scratch, size_t scratch_bytes) {
   if (int rc = check_delta("delta_scan", d, rows)) return rc;
   GRETA_REQUIRE(!rows->d_pos && o_buf && d->r && d->k && d->v && d->a && d->decay && d->state, "delta_scan: null pointer, or rows of a batch");
   GRETA_REQUIRE(aligned16(d->state), "delta_scan: misaligned state");
-  return pick_scan<false>((cudaStream_t)stream, ScanArgs{d->decay, d->k, d->a, d->r, d->v, d->ld_decay, d->ld, d->ld, d->ld, d->ld, d->heads, 1, d->dim, d->dim,
-                                                        rows->M, rows->pos0, rows->slot0, d->state}, o_buf);
+  return scan<false>((cudaStream_t)stream, ScanArgs{d->decay, d->k, d->a, d->r, d->v, d->ld_decay, d->ld, d->ld, d->ld, d->ld, d->heads, 1, d->dim, d->dim,
+                                                   rows->M, rows->pos0, rows->slot0, d->state}, o_buf, scratch, scratch_bytes);
 }
 
 int greta_cuda_delta_output(greta_stream_t stream, const greta_delta_rule *d, const float *o_buf, uint32_t M, void *out, int out_fmt, uint32_t ld_out) {
@@ -865,11 +858,19 @@ int greta_cuda_gated_delta_prepare(greta_stream_t stream, const greta_gated_delt
 }
 
 int greta_cuda_gated_delta_scan(greta_stream_t stream, const greta_gated_delta *d, const greta_rows *rows, float *o_buf) {
+  return greta_cuda_gated_delta_scan_chunked(stream, d, rows, o_buf, nullptr, 0);
+}
+size_t greta_cuda_gated_delta_scan_scratch_bytes(uint32_t heads, uint32_t dim, uint32_t vdim, uint32_t rows) {
+  return chunk_scan_bytes(heads, dim, vdim, true, rows);
+}
+int greta_cuda_gated_delta_scan_chunked(greta_stream_t stream, const greta_gated_delta *d, const greta_rows *rows, float *o_buf, void *scratch,
+                                        size_t scratch_bytes) {
   if (int rc = check_gated("gated_delta_scan", d, rows)) return rc;
   GRETA_REQUIRE(!rows->d_pos && o_buf && d->u && d->beta && d->decay, "gated_delta_scan: null pointer, or rows of a batch");
   const uint32_t GD = d->kv_heads * d->dim;
-  return pick_scan<true>((cudaStream_t)stream, ScanArgs{d->decay, d->u + GD, d->beta, d->u, d->u + 2 * GD, d->ld_decay, d->ld_u, d->ld_beta, d->ld_u, d->ld_u,
-                                                       d->heads, d->heads / d->kv_heads, d->dim, d->vdim, rows->M, rows->pos0, rows->slot0, d->state}, o_buf);
+  return scan<true>((cudaStream_t)stream, ScanArgs{d->decay, d->u + GD, d->beta, d->u, d->u + 2 * GD, d->ld_decay, d->ld_u, d->ld_beta, d->ld_u, d->ld_u,
+                                                  d->heads, d->heads / d->kv_heads, d->dim, d->vdim, rows->M, rows->pos0, rows->slot0, d->state},
+                    o_buf, scratch, scratch_bytes);
 }
 
 int greta_cuda_gated_delta_output(greta_stream_t stream, const greta_gated_delta *d, const float *o_buf, uint32_t M, void *out, int out_fmt, uint32_t ld_out) {

@@ -339,7 +339,7 @@ bool BlockScheduler::allocate_hybrid_activations(std::string *err) {
     return true;
   };
   uint32_t proj = 4, cat = 64, q = 4, o = 4, low = 0, low16 = 0, hd = 0, q_latent = 0, u = 0, gate = 0;
-  size_t scratch = 0, qx = 0, kx = 0, vx = 0;
+  size_t scratch = 0, scan = 0, qx = 0, kx = 0, vx = 0;
   const uint32_t absorbed = bf16 ? std::max(B, std::min(chunk, MMA_MIN_ROWS - 1)) : R;  // rows that latent attention takes in its absorbed form
   for (uint32_t l = 0; l < c.num_layers; ++l) {
     const MixerSpec &m = c.layers[l].mixer;
@@ -352,6 +352,7 @@ bool BlockScheduler::allocate_hybrid_activations(std::string *err) {
         low = std::max(low, m.rank);
         low16 = std::max(low16, 2 * up(m.rank, 8));
         hd = std::max(hd, HD);
+        scan = std::max(scan, greta_cuda_delta_scan_scratch_bytes(m.heads, m.dim, R));
         break;
       case MixerKind::GATED_DELTA:
         o = std::max(o, m.out_cols());
@@ -360,6 +361,7 @@ bool BlockScheduler::allocate_hybrid_activations(std::string *err) {
         hd = std::max(hd, HD);
         u = std::max(u, up(m.conv_cols(), 4));
         gate = std::max(gate, up(m.out_cols(), 4));
+        scan = std::max(scan, greta_cuda_gated_delta_scan_scratch_bytes(m.heads, m.dim, m.vdim, R));
         break;
       case MixerKind::LATENT_ATTENTION: {
         q = std::max(q, m.q_cols());
@@ -398,7 +400,7 @@ bool BlockScheduler::allocate_hybrid_activations(std::string *err) {
               !zeroed(w.decay, (size_t)R * w.decay_ld * 4) || !zeroed(w.o, (size_t)R * o * 4)))
     return false;
   if ((u && (!zeroed(w.u, (size_t)R * u * 4) || !zeroed(w.gate, (size_t)R * gate * 4))) || (q_latent && !zeroed(w.q_latent, (size_t)R * q_latent * cb)) ||
-      (scratch && !zeroed(w.latent_scratch, scratch)) || (kx && (!zeroed(w.q_tiles, qx, GretaDataType::FP16) || !zeroed(w.k_expanded, kx, GretaDataType::FP16) || !zeroed(w.v_expanded, vx, GretaDataType::FP16))))
+      (scratch && !zeroed(w.latent_scratch, scratch)) || (scan && !zeroed(w.scan_scratch, scan)) || (kx && (!zeroed(w.q_tiles, qx, GretaDataType::FP16) || !zeroed(w.k_expanded, kx, GretaDataType::FP16) || !zeroed(w.v_expanded, vx, GretaDataType::FP16))))
     return false;
   rotation_tables_ = std::vector<Buffer>(rotations_.size());
   for (size_t r = 0; r < rotations_.size(); ++r) {  // angles in double: the tables are as exact as their fp32 entries
@@ -624,7 +626,7 @@ bool BlockScheduler::general_delta_core(size_t layer, const greta_rows &rows, st
     GRETA_TRY(greta_cuda_linear_gemv(s, &dec, low, w.low_ld, nullptr, nullptr, 0.f, rows.M), "decay");
   else
     GRETA_TRY(greta_cuda_linear_gemm(s, &dec, low_pair ? w.low16.data() : w.low.data(), low_pair ? w.low16_ld : w.low_ld, rows.M), "decay");
-  GRETA_TRY(greta_cuda_delta_scan(s, &d, &rows, static_cast<float *>(w.o.data())), "delta scan");
+  GRETA_TRY(greta_cuda_delta_scan_chunked(s, &d, &rows, static_cast<float *>(w.o.data()), w.scan_scratch.data(), w.scan_scratch.size()), "delta scan");
   GRETA_TRY(greta_cuda_delta_output(s, &d, fp(w.o), rows.M, cat, cat_fmt, w.cat_ld), "delta output");
   return true;
 }
@@ -789,7 +791,7 @@ bool BlockScheduler::gated_delta_core(size_t layer, const greta_rows &rows, std:
   else
     GRETA_TRY(greta_cuda_linear_gemm(s, &low2, low_pair ? w.low16.data() : w.low.data(), low_pair ? w.low16_ld : w.low_ld, rows.M), "decay and gate");
   GRETA_TRY(greta_cuda_gated_delta_prepare(s, &d, &rows), "delta inputs");
-  GRETA_TRY(greta_cuda_gated_delta_scan(s, &d, &rows, static_cast<float *>(w.o.data())), "delta scan");
+  GRETA_TRY(greta_cuda_gated_delta_scan_chunked(s, &d, &rows, static_cast<float *>(w.o.data()), w.scan_scratch.data(), w.scan_scratch.size()), "delta scan");
   GRETA_TRY(greta_cuda_gated_delta_output(s, &d, fp(w.o), rows.M, cat, cat_fmt, w.cat_ld), "delta output");
   return true;
 }

@@ -624,6 +624,12 @@ GRETA_API size_t greta_cuda_delta_state_bytes(uint32_t heads, uint32_t dim); /* 
 GRETA_API int greta_cuda_delta_step(greta_stream_t stream, const greta_delta_rule *d, const greta_rows *rows, void *out, int out_fmt, uint32_t ld_out);
 /* A portion: the recurrence over its rows, o -> o_buf fp32 [M][heads*dim]; then norm and gate. */
 GRETA_API int greta_cuda_delta_scan(greta_stream_t stream, const greta_delta_rule *d, const greta_rows *rows, float *o_buf);
+/* The same, 16 tokens at a time through scratch (16-byte aligned).  scratch_bytes: for portions of at most that many rows; 0: the form does
+ * not cover the sizes (it takes dim32 of 64 and 128) or the rows are too few.  A call that it does not cover, or whose scratch is
+ * too small, runs as greta_cuda_delta_scan. */
+GRETA_API size_t greta_cuda_delta_scan_scratch_bytes(uint32_t heads, uint32_t dim, uint32_t rows);
+GRETA_API int greta_cuda_delta_scan_chunked(greta_stream_t stream, const greta_delta_rule *d, const greta_rows *rows, float *o_buf, void *scratch,
+                                            size_t scratch_bytes);
 GRETA_API int greta_cuda_delta_output(greta_stream_t stream, const greta_delta_rule *d, const float *o_buf, uint32_t M, void *out, int out_fmt,
                                       uint32_t ld_out);
 
@@ -665,6 +671,10 @@ GRETA_API int greta_cuda_gated_delta_step(greta_stream_t stream, const greta_gat
  * norm and gate. */
 GRETA_API int greta_cuda_gated_delta_prepare(greta_stream_t stream, const greta_gated_delta *d, const greta_rows *rows);
 GRETA_API int greta_cuda_gated_delta_scan(greta_stream_t stream, const greta_gated_delta *d, const greta_rows *rows, float *o_buf);
+/* As greta_cuda_delta_scan_chunked. */
+GRETA_API size_t greta_cuda_gated_delta_scan_scratch_bytes(uint32_t heads, uint32_t dim, uint32_t vdim, uint32_t rows);
+GRETA_API int greta_cuda_gated_delta_scan_chunked(greta_stream_t stream, const greta_gated_delta *d, const greta_rows *rows, float *o_buf, void *scratch,
+                                                  size_t scratch_bytes);
 GRETA_API int greta_cuda_gated_delta_output(greta_stream_t stream, const greta_gated_delta *d, const float *o_buf, uint32_t M, void *out, int out_fmt,
                                             uint32_t ld_out);
 
