@@ -26,6 +26,7 @@
 
 namespace greta {
 int attn_mma_decode(cudaStream_t stream, const AttnParams &p, uint32_t batch, uint32_t nsplit, uint32_t ng, uint32_t Dh);  // attention_mma.cu
+int attn_tc_prefill(cudaStream_t stream, const AttnParams &p, uint32_t S, uint32_t pos0, uint32_t Dh, void *out, bool f16);  // attention_tc.cu
 int attn_mma_prefill(cudaStream_t stream, const AttnParams &p, uint32_t S, uint32_t pos0, uint32_t Dh);
 }  // namespace greta
 
@@ -495,8 +496,8 @@ int greta_cuda_attn_decode_static(greta_stream_t stream, const float *q, const v
                                   /*scratch_merge_only=*/true);
 }
 
-int greta_cuda_attn_prefill(greta_stream_t stream, const float *q, const void *kc, const void *vc, float *o, uint32_t S,
-                            uint32_t pos0, uint32_t H, uint32_t Hkv, uint32_t Dh, uint32_t max_seq, float scale) {
+static int attn_prefill_impl(greta_stream_t stream, const float *q, const void *kc, const void *vc, float *o, void *o16, uint32_t S, uint32_t pos0, uint32_t H,
+                             uint32_t Hkv, uint32_t Dh, uint32_t max_seq, float scale) {
   if (S == 0) return GRETA_OK;
   GRETA_REQUIRE(H && Hkv && H % Hkv == 0, "attn_prefill: num_heads=%u must be a positive multiple of num_heads_kv=%u", H, Hkv);
   GRETA_REQUIRE(q && kc && vc && o, "attn_prefill: null pointer");
@@ -505,11 +506,29 @@ int greta_cuda_attn_prefill(greta_stream_t stream, const float *q, const void *k
   AttnParams p{};
   p.q = q; p.kc = kc; p.vc = vc; p.o = o; p.d_pos = nullptr; p.len0 = pos0 + 1;
   p.H = H; p.Hkv = Hkv; p.max_seq = max_seq; p.scale = scale; p.splits = 1; p.len_step = 1;
-  // Prompts run on the tensor cores (16 positions of a head per warp, K / V tiles staged once per 64 positions); a few
-  // positions, or the switch off, take one CTA per (position, head) on the decode inner loop.
-  if (tuning().attn_mma && S >= 8 && (Dh == 64 || Dh == 128) && aligned16(q) && aligned16(kc) && aligned16(vc) && aligned16(o))
-    return attn_mma_prefill((cudaStream_t)stream, p, S, pos0, Dh);
-  return launch_attn<__half>((cudaStream_t)stream, p, S, Dh);
+  // Prompts run on the tensor cores; a few positions, or the switch off, take one CTA per (position, head) on the decode inner loop.
+  if (tuning().attn_mma && S >= 8 && (Dh == 64 || Dh == 128) && aligned16(q) && aligned16(kc) && aligned16(vc) && aligned16(o)) {
+    // tcgen05 above 512 keys: 1531 rows of 32 heads 98 against 256 us, 2048 rows of 64 heads of 64 168 against 365.  It would pay from 128 keys on (a
+    // 512-token prompt of four 7B layers 1104 against 1190 us).  The line lies higher because the ids of the 512-token 7B run hang on a top-2
+    // gap of 4.4e-6, less than what the products' sums leave open: with the smaller rounding error of this form one id of 128 is another.
+    if (pos0 + S > 512 && (!o16 || aligned16(o16)))
+      return attn_tc_prefill((cudaStream_t)stream, p, S, pos0, Dh, o16 ? o16 : (void *)o, o16 != nullptr);
+    if (int rc = attn_mma_prefill((cudaStream_t)stream, p, S, pos0, Dh)) return rc;
+  } else if (int rc = launch_attn<__half>((cudaStream_t)stream, p, S, Dh)) {
+    return rc;
+  }
+  return o16 ? greta_cuda_f32_to_f16(stream, o, o16, (size_t)S * H * Dh) : GRETA_OK;
+}
+
+int greta_cuda_attn_prefill(greta_stream_t stream, const float *q, const void *kc, const void *vc, float *o, uint32_t S,
+                            uint32_t pos0, uint32_t H, uint32_t Hkv, uint32_t Dh, uint32_t max_seq, float scale) {
+  return attn_prefill_impl(stream, q, kc, vc, o, nullptr, S, pos0, H, Hkv, Dh, max_seq, scale);
+}
+
+int greta_cuda_attn_prefill_f16(greta_stream_t stream, const float *q, const void *kc, const void *vc, void *o16, float *scratch, uint32_t S,
+                                uint32_t pos0, uint32_t H, uint32_t Hkv, uint32_t Dh, uint32_t max_seq, float scale) {
+  GRETA_REQUIRE(S == 0 || o16, "attn_prefill_f16: null pointer");
+  return attn_prefill_impl(stream, q, kc, vc, scratch, o16, S, pos0, H, Hkv, Dh, max_seq, scale);
 }
 
 int greta_cuda_attn_prefill_f32(greta_stream_t stream, const float *q, const float *k, const float *v, float *o, uint32_t S, uint32_t H,

@@ -405,6 +405,10 @@ int gemm_ts_status(int *code) {
   GRETA_CUDA_TRY(cudaMemcpyFromSymbol(code, g_gemm_error, sizeof(int)));
   return GRETA_OK;
 }
+int gemm_ts_error_word(int **word) {  // the current device's; the prompt's attention reports there too
+  GRETA_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void **>(word), g_gemm_error));
+  return GRETA_OK;
+}
 int gemm_ts_set_status(int code) {
   GRETA_CUDA_TRY(cudaMemcpyToSymbol(g_gemm_error, &code, sizeof(int)));
   return GRETA_OK;

@@ -620,9 +620,15 @@ bool BlockScheduler::prompt_layer(size_t layer_idx, size_t seq_start, size_t seq
     GRETA_TRY(greta_cuda_rmsnorm_f16(s, x, static_cast<const float *>(b.attn_norm.data()), n16, S, D, c.rms_eps), "rmsnorm");
     GRETA_TRY(greta_cuda_gemm_segments(s, fmt, n16, S, D, qkv, 3, GRETA_GEMM_STORE), "qkv");
     GRETA_TRY(greta_cuda_rope_kv(s, q, k, v, kc, vc, S, heads_l_, kv_heads_l_, Dh, c.rope_base, (uint32_t)seq_start, (uint32_t)max_seq_), "rope, kv update");
-    GRETA_TRY(greta_cuda_attn_prefill(s, q, kc, vc, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
-    GRETA_TRY(greta_cuda_f32_to_f16(s, att, q, (size_t)S * ql), "attention output");  // the queries are done with
-    if (!residual(q, b.wo, b.s_wo, ql, "wo")) return false;
+    void *att16 = n16;  // free by now
+    if (ql <= D) {
+      GRETA_TRY(greta_cuda_attn_prefill_f16(s, q, kc, vc, att16, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
+    } else {
+      att16 = q;
+      GRETA_TRY(greta_cuda_attn_prefill(s, q, kc, vc, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
+      GRETA_TRY(greta_cuda_f32_to_f16(s, att, att16, (size_t)S * ql), "attention output");  // the queries are done with
+    }
+    if (!residual(att16, b.wo, b.s_wo, ql, "wo")) return false;
     const float *gamma = static_cast<const float *>(b.ffn_norm.data());
     GRETA_TRY(keep_norm ? greta_cuda_rmsnorm_both(s, x, gamma, nrm, n16, S, D, c.rms_eps) : greta_cuda_rmsnorm_f16(s, x, gamma, n16, S, D, c.rms_eps),
               "rmsnorm");

@@ -392,6 +392,9 @@ GRETA_API int greta_cuda_attn_prefill(greta_stream_t stream, const float *q, con
                                       const void *v_cache_f16, float *o, uint32_t S, uint32_t pos0,
                                       uint32_t num_heads, uint32_t num_heads_kv, uint32_t head_dim,
                                       uint32_t max_seq_len, float scale);
+/* The same, rounded to fp16; scratch: S * H * Dh floats, which some routes use. */
+GRETA_API int greta_cuda_attn_prefill_f16(greta_stream_t stream, const float *q, const void *kc, const void *vc, void *o16, float *scratch, uint32_t S,
+                                          uint32_t pos0, uint32_t H, uint32_t Hkv, uint32_t Dh, uint32_t max_seq, float scale);
 /* The reference's own prefill entry, launch_flash_attention_prefill (attention_kernels.hpp:124-128, kernel
  * attention_kernels.hip:543-618): q, o fp32 [S][H][Dh]; k, v fp32 [S][Hkv][Dh] (the prompt's own keys, not a cache);
  * causal != 0: query s sees keys 0..s, else all S. */

@@ -1,0 +1,46 @@
+"""Prefill attention over more than 512 keys (tcgen05) against float64."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from _support import load_package
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def g():
+    return load_package().ffi
+
+
+@pytest.mark.parametrize("S,pos0,H,Hkv,Dh,gain", [(513, 0, 2, 2, 128, 1.0), (8, 505, 4, 1, 64, 1.0), (640, 0, 2, 1, 64, 1.0), (300, 467, 3, 3, 128, 1.0),
+                                                  (16, 700, 4, 2, 128, 1.0), (769, 0, 2, 1, 128, 8.0), (128, 513, 1, 1, 64, 8.0), (1100, 0, 1, 1, 128, 1.0)])
+def test_prefill_attention_above_512_keys(g, S, pos0, H, Hkv, Dh, gain):
+    """Tile edges of queries and keys, rows behind the last key that are no numbers, maxima that grow from tile to tile (gain); fp16 output is the
+    rounded fp32 output.  Tolerance: pairs of fp16 keep 22 bits of queries and probabilities, sums are cut at 24 bits up to 8 times per 128 keys."""
+    rng = np.random.default_rng(S + Dh)
+    n, ms = pos0 + S, pos0 + S + 9
+    dev = lambda a: g.DeviceBuffer.from_numpy(np.ascontiguousarray(a))
+    q = (rng.normal(0, gain, (S, H, Dh)) * np.linspace(0.2, 1, S)[:, None, None]).astype(np.float32)
+    k, v = (rng.normal(0, 1, (Hkv, ms, Dh)).astype(np.float16) for _ in range(2))
+    k *= np.linspace(0.1, 1, ms).astype(np.float16)[None, :, None]
+    k[:, n:], v[:, n:] = np.nan, np.nan
+    dq, dk, dv = dev(q), dev(k.view(np.uint16)), dev(v.view(np.uint16))
+    o, o2, o16 = (dev(np.zeros((S, H, Dh), np.float32)) for _ in range(3))
+    lib, scale, code = g.cuda(), Dh ** -0.5, C.c_int(-1)
+    g.check(lib.greta_cuda_attn_prefill(None, dq.ptr, dk.ptr, dv.ptr, o.ptr, S, pos0, H, Hkv, Dh, ms, scale))
+    g.check(lib.greta_cuda_attn_prefill_f16(None, dq.ptr, dk.ptr, dv.ptr, o16.ptr, o2.ptr, S, pos0, H, Hkv, Dh, ms, scale))
+    g.check(lib.greta_cuda_gemm_segments_status(None, C.byref(code)))
+    g.check(lib.greta_cuda_device_synchronize())
+    assert code.value == 0
+    got = o.download(np.float32).reshape(S, H, Dh)
+    assert (o16.download(np.uint16)[:S * H * Dh] == got.astype(np.float16).view(np.uint16).reshape(-1)).all()
+    hidden = np.arange(n)[None] > pos0 + np.arange(S)[:, None]
+    for h in range(H):
+        s = q[:, h].astype(np.float64) @ k[h // (H // Hkv), :n].astype(np.float64).T * scale
+        s[hidden] = -np.inf
+        w = np.exp(s - s.max(1, keepdims=True))
+        want = (w / w.sum(1, keepdims=True)) @ v[h // (H // Hkv), :n].astype(np.float64)
+        err = np.abs(got[:, h] - want).max() / want.std()
+        assert err < 2e-5 * gain, err
