@@ -607,14 +607,17 @@ struct PPlan {
   // CTAs per SM this plan fits: the most that the format aims at and that leaves a weight ring of at least two stages
   static constexpr int CTAS = (PFmt<FMT>::CTAS_PER_SM >= 3 && room_in(74 * 1024, 1) >= 2) ? 3 : ((PFmt<FMT>::CTAS_PER_SM >= 2 && room_in(112 * 1024, 1) >= 2) ? 2 : 1);
   static constexpr int LIMIT = CTAS == 3 ? 74 * 1024 : (CTAS == 2 ? 112 * 1024 : (int)BSMEM_LIMIT);
-  // Two activation buffers of XCELLS cells each; a buffer is refilled XCELLS cells ahead, which the weight ring must
-  // cover: XCELLS <= DEPTH - 1.  Two CTAs of 8 warps per SM (128 rows each) balance the SMs better than one of 16.
+  // Two activation buffers of XCELLS cells each; a buffer is refilled XCELLS cells ahead.  Two CTAs of 8 warps per SM (128
+  // rows each) balance the SMs better than one of 16.
   static constexpr int room(int xcells) { return room_in(LIMIT, xcells); }
   static constexpr int XCELLS = (MT < 4 && room(2) >= 3) ? 2 : 1;
   static constexpr int DEPTH = room(XCELLS) > 4 ? 4 : room(XCELLS);
   static constexpr int XBUF = XCELLS * CELL * MT * 1024;
   static constexpr size_t SMEM = (size_t)2 * XBUF + ROWTAB + (size_t)NW * DEPTH * STAGE;
-  static_assert(DEPTH >= 2 && XCELLS <= DEPTH - 1, "shared memory plan");
+  // A cell commits its activations and its weights as two groups, in this order.  The weights a cell reads were committed DEPTH - 1 cells
+  // before it, 2 (DEPTH - 2) groups from the end; the activations XCELLS cells before it, 2 XCELLS - 1 groups from the end.
+  static constexpr int PENDING = 2 * (DEPTH - 2) < 2 * XCELLS - 1 ? 2 * (DEPTH - 2) : 2 * XCELLS - 1;
+  static_assert(DEPTH >= 2, "shared memory plan");
 };
 
 __device__ __forceinline__ void mma_f16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -624,8 +627,8 @@ __device__ __forceinline__ void mma_f16_first(float (&d)[4], uint32_t a0, uint32
 }
 
 // The matmul on prepared activations: NW warps, one 16-row tile per warp, K split over the cluster as above.  All warps
-// walk the cells of the slice in step; the prepared activations of the next cells arrive by cp.async in the same commit
-// groups as the weight cells, one CTA-wide barrier per activation buffer.
+// walk the cells of the slice in step; the prepared activations of the next cells arrive by cp.async between the weight
+// cells, one CTA-wide barrier per activation buffer.
 template <int FMT, int EPI, int MT>
 __global__ void __launch_bounds__(PFmt<FMT>::NW * 32, PPlan<FMT, MT>::CTAS) gemv_batchp_kernel(const GemvParams p) {
   using F = BFmt<FMT>;
@@ -712,7 +715,7 @@ __global__ void __launch_bounds__(PFmt<FMT>::NW * 32, PPlan<FMT, MT>::CTAS) gemv
     if (c == cs)
       cp_async_wait(0);  // the first activation chunk is the newest group
     else
-      cp_async_wait_c<DEPTH - 2>();
+      cp_async_wait_c<P::PENDING>();
     const uint32_t rel = c - cs, chunk = rel / XCELLS;
     if (rel % XCELLS == 0) {
       __syncthreads();  // everybody's pieces of this chunk are in; everybody is done with the chunk before
@@ -720,6 +723,7 @@ __global__ void __launch_bounds__(PFmt<FMT>::NW * 32, PPlan<FMT, MT>::CTAS) gemv
     } else {
       __syncwarp();
     }
+    cp_async_commit();
     request_weights();
     cp_async_commit();
     const uint8_t *st = myring + cstage * STAGE;

@@ -1,0 +1,31 @@
+"""The batched matmul on prepared activations waits for the activations of a cell as well as for its weights: with the caches cold and few rows,
+cells are multiplied faster than the next cell's activations arrive."""
+import numpy as np
+import pytest
+
+from _support import load_package
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 32000, 4096), (1, 32000, 2048), (16, 32000, 4096)])
+def test_activations_have_landed_before_they_are_read(M, N, K):
+    g = load_package().ffi
+    lib, rng = g.cuda(), np.random.default_rng(M)
+    w = (rng.standard_normal((N, K), dtype=np.float32) * 0.02).astype(np.float16)
+    rows = np.arange(0, N, 97)
+    flush = g.DeviceBuffer(256 << 20)
+    dw, y = g.DeviceBuffer.from_numpy(w.view(np.uint16)), g.DeviceBuffer(M * N * 4)
+    ws = g.DeviceBuffer(lib.greta_cuda_gemv_batch_workspace_bytes(M, K))
+    for i in range(4):                                        # other activations each time: what lay there before does not do
+        x = rng.standard_normal((M, K), dtype=np.float32)
+        dx = g.DeviceBuffer.from_numpy(x)
+        flush.fill(i)
+        g.check(lib.greta_cuda_gemv_batch(None, g.FMT_F16, dx.ptr, None, 0.0, dw.ptr, None, None, y.ptr, M, N, K, 0, ws.ptr))
+        g.check(lib.greta_cuda_device_synchronize())
+        want = x.astype(np.float64) @ w[rows].astype(np.float64).T
+        got = y.download(np.float32).reshape(M, N)[:, rows]
+        # K products of exact weights and 22-bit activations, summed in fp32 over at most 128 blocks and 8 slices
+        assert np.abs(got - want).max() < 2e-5 * np.abs(want).max(), i
+    for b in (flush, dw, y, ws):
+        b.free()
