@@ -35,6 +35,7 @@
 #include <algorithm>
 
 #include "gemv_device.cuh"
+#include "gemv_tc.cuh"
 
 namespace {
 
@@ -892,6 +893,7 @@ int launch_batch(cudaStream_t stream, const GemvParams &p, void *workspace = nul
 template <int EPI>
 int dispatch_batch(cudaStream_t stream, int fmt, const GemvParams &p, void *workspace = nullptr) {
   GRETA_REQUIRE(!workspace || aligned16(workspace), "batched gemv: the workspace must be 16-byte aligned");
+  if (workspace && p.kw == 0 && gemv_tc_takes(fmt, EPI, &p)) return gemv_tc(stream, fmt, EPI, &p, workspace);
   switch (fmt) {
     case GRETA_FMT_Q4_0: return launch_batch<GRETA_FMT_Q4_0, EPI>(stream, p, workspace);
     case GRETA_FMT_Q8_0: return launch_batch<GRETA_FMT_Q8_0, EPI>(stream, p, workspace);
@@ -937,7 +939,7 @@ extern "C" {
 
 size_t greta_cuda_gemv_batch_workspace_bytes(uint32_t M, uint32_t K) {
   const size_t mt = M <= 8 ? 1 : (M <= 16 ? 2 : 4);
-  return PREP_HEADER + (size_t)(K / 32) * mt * 1024;
+  return std::max(PREP_HEADER + (size_t)(K / 32) * mt * 1024, gemv_tc_workspace_bytes(M, K));
 }
 
 int greta_cuda_gemv_batch(greta_stream_t stream, int fmt, const float *x, const float *gamma, float eps, const void *qs, const void *d,

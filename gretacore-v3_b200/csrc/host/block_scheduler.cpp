@@ -174,7 +174,8 @@ bool BlockScheduler::allocate_activations(size_t batch_size, size_t max_seq_len,
   if (!dev(a.x, S * D * 4) || !dev(a.norm_out, S * D * 4) || !dev(a.q, S * ql * 4) || !dev(a.k, S * kvl * 4) || !dev(a.v, S * kvl * 4) ||
       !dev(a.attn_out, S * ql * 4) || !dev(a.mlp_gate, S * hidden_l_ * 4) || !dev(a.mlp_up, few * hidden_l_ * 4) || !dev(a.mlp_out, (c.tp_size > 1 ? S : few) * D * 4))
     return false;
-  if (S > SKINNY_ROWS && (!dev(a.norm_f16, S * D * 2, GretaDataType::FP16) || !a.gave_up.allocate(16, BufferUsage::HostVisible, GretaDataType::FP32, err))) return false;
+  if (S > SKINNY_ROWS && !dev(a.norm_f16, S * D * 2, GretaDataType::FP16)) return false;
+  if ((S > SKINNY_ROWS || B > 1) && !a.gave_up.allocate(16, BufferUsage::HostVisible, GretaDataType::FP32, err)) return false;
   const size_t cache = (size_t)c.num_layers * B * kv_heads_l_ * max_seq_len * c.head_dim * 2;  // [L][B][Hkv][S][Dh] fp16
   if (!dev(a.kv_cache_k, cache, GretaDataType::FP16) || !dev(a.kv_cache_v, cache, GretaDataType::FP16)) return false;
   // d_pos: B positions, then B counts of ids produced; d_next: B token ids; out_tokens: [B][max_seq]
@@ -690,14 +691,19 @@ bool BlockScheduler::forward(const int32_t *tokens, size_t seq_start, size_t seq
   }
   if (!lm_head(static_cast<const float *>(a.x.data()) + (seq_len - 1) * c.dim, err)) return false;
   int *gave_up = seq_len > SKINNY_ROWS ? static_cast<int *>(a.gave_up.data()) : nullptr;
-  if (gave_up) GRETA_TRY(greta_cuda_gemm_segments_status(s, gave_up), "forward");
-  GRETA_TRY(greta_cuda_stream_synchronize(s), "forward");
-  if (gave_up && *gave_up) {  // results and cache rows are wrong; the code is reported once
-    const int code = *gave_up;
-    greta_cuda_gemm_set_status(0);
-    return fail(err, "forward: a bounded wait of a prompt product gave up (code " + std::to_string(code) + ")");
-  }
-  return true;
+  return products_finished(gave_up, "forward", "prompt", err);
+}
+
+// Waits for the stream, and fails where a bounded wait of a tensor-core product gave up: results and cache rows are wrong then; the code is
+// reported once.  `gave_up` is page-locked, or null where the work had no such products.
+bool BlockScheduler::products_finished(int *gave_up, const char *what, const char *kind, std::string *err) {
+  cudaStream_t s = H(stream_);
+  if (gave_up) GRETA_TRY(greta_cuda_gemm_segments_status(s, gave_up), what);
+  GRETA_TRY(greta_cuda_stream_synchronize(s), what);
+  if (!gave_up || !*gave_up) return true;
+  const int code = *gave_up;
+  greta_cuda_gemm_set_status(0);
+  return fail(err, std::string(what) + ": a bounded wait of a " + kind + " product gave up (code " + std::to_string(code) + ")");
 }
 
 bool BlockScheduler::forward_logits(const int32_t *tokens, size_t seq_start, size_t seq_len, const uint32_t *rows, size_t n_rows, float *out,
@@ -901,13 +907,13 @@ bool BlockScheduler::decode_step_host(const int32_t *token_in, int32_t *token_ou
   GRETA_TRY(greta_cuda_memcpy_h2d(activations_.d_next.data(), token_in, (size_t)batch_ * 4, s), "token upload");
   if (graph_->launch(stream_) != gcore::rt::GretaResult::SUCCESS) return fail(err, gcore::host::cuda_error("decode step launch failed"));
   GRETA_TRY(greta_cuda_memcpy_d2h(token_out, activations_.d_next.data(), (size_t)batch_ * 4, s), "token download");
-  GRETA_TRY(greta_cuda_stream_synchronize(s), "decode_step_host");
+  if (!products_finished(batch_ > 1 ? static_cast<int *>(activations_.gave_up.data()) : nullptr, "decode_step_host", "batch", err)) return false;
   ++decode_steps_;
   return true;
 }
 
 bool BlockScheduler::read_generated(int32_t *out, size_t n, std::string *err) {
-  GRETA_TRY(greta_cuda_stream_synchronize(H(stream_)), "read_generated");
+  if (!products_finished(batch_ > 1 ? static_cast<int *>(activations_.gave_up.data()) : nullptr, "read_generated", "batch", err)) return false;
   if (n > decode_steps_) return fail(err, "read_generated: fewer steps were run");
   // out is [batch][n]; the device list is [batch][max_seq].  One strided copy: a copy per sequence cost 7 us each.
   return activations_.out_tokens.copy_rows_to_host(out, (size_t)max_seq_ * 4, n * 4, batch_, err);

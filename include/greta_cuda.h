@@ -231,9 +231,10 @@ GRETA_API int greta_cuda_fused_ffn_front(greta_stream_t stream, int fmt, const f
  * 16-byte aligned; outputs are [M][...] row-major.  k_slices forces the number of K slices (1, 2, 4 or 8; 0 =
  * chosen from the shape).
  * workspace: greta_cuda_gemv_batch_workspace_bytes(M, K) bytes of device memory, 16-byte aligned, or NULL.  With it the
- * activations are converted once, by a small kernel in front, into the layout the tensor-core kernel consumes; without
- * it every CTA of the matmul kernel repeats that conversion for itself (about 2.5 times slower, same results to the
- * last bit of the fp16 pairs).  One workspace can serve every call on a stream.
+ * activations are converted once, by a small kernel in front, into the layout the tensor-core kernel consumes, and large
+ * products (k_slices 0) go through tcgen05: their weights reach the tensor cores through tensor memory, row tiles that
+ * several CTAs share are summed in the workspace.  Without it every CTA of the matmul kernel repeats that conversion for
+ * itself.  One workspace can serve every call on a stream, one call at a time.
  *
  * y[M][N] = (resid ? resid[M][N] : 0) + rmsnorm?(x)[M][K] * dequant(W)^T; gamma == NULL: no norm. */
 GRETA_API size_t greta_cuda_gemv_batch_workspace_bytes(uint32_t M, uint32_t K);
@@ -333,7 +334,7 @@ GRETA_API int greta_cuda_gemm_segments(greta_stream_t stream, int fmt, const voi
  * memory, tiles of the launch (one persistent CTA per SM goes through them). */
 GRETA_API int greta_cuda_gemm_segments_route(uint32_t M, uint32_t K, const uint32_t *n, uint32_t n_segs, int mode, uint32_t *tile_tokens,
                                              uint32_t *accumulators, uint32_t *weight_slots, uint32_t *tiles);
-/* The code of its kernels so far on the stream: valid in *code once the stream has been synchronised (*code in page-locked memory). */
+/* The code of its kernels, of the prompt's attention and of the batched products so far on the stream: valid in *code once the stream has been synchronised (*code in page-locked memory). */
 GRETA_API int greta_cuda_gemm_segments_status(greta_stream_t stream, int *code);
 
 /* ------------------------------------------------------------------ attention
