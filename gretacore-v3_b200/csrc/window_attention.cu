@@ -467,17 +467,24 @@ struct MmaCfg {
   static constexpr size_t SMEM = (size_t)(WM_Q + 4 * WM_K) * ROWP;
 };
 
-// grid (query tiles, heads); DB: head size bucket (64, 128 or 256) for both dim and vdim, unused columns zero.
+// One CTA per query tile and head; DB: head size bucket (64, 128 or 256) for both dim and vdim, unused columns zero.
+// What bounds it: per score the special-function unit makes three results (soft cap: 2^x and a reciprocal; the weight: 2^x), 24 cycles per 32
+// scores, and the matrix instructions take about as long.  The logarithm of the distance comes from a table of `tab` distances in shared
+// memory (a fourth result and a conversion otherwise), and tiles whose keys every row sees, all but three or four of a row's, skip positions and
+// masks.  Measured at 2048
+// rows of 32 heads of 64 behind a window of 1024 and 64 kept positions, caches cold: 197 us before the table and the short path, 166 with them, 138 with
+// one thread's copies in one column (divisions by the row's length before) and no rescaling by 1, 132 with four CTAs per SM, 112 with the longest
+// rows of all heads first (before: of each head).  Special-function unit 43 % busy, tensor pipe 26 %, issue slots 47 %.
 template <int DB>
-__global__ void __launch_bounds__(WM_THREADS) window_mma_kernel(const __grid_constant__ WinArgs w, const float *q_in, void *out, int out_fmt,
-                                                                uint32_t ld_out) {
+__global__ void __launch_bounds__(WM_THREADS, DB == 64 ? 4 : (DB == 128 ? 2 : 1)) window_mma_kernel(const __grid_constant__ WinArgs w, const float *q_in, void *out, int out_fmt,
+                                                                uint32_t ld_out, uint32_t tab) {
   constexpr int ROWP = MmaCfg<DB>::ROWP;
   constexpr float LOG2E = 1.4426950408889634f;
   extern __shared__ __align__(16) uint8_t smb[];
   uint8_t *qs = smb, *kt = qs + WM_Q * ROWP, *vt = kt + 2 * WM_K * ROWP;  // two K tiles, two V tiles
   const greta_window_attn &a = w.a;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3, mat = lane >> 3, r8 = lane & 7;
-  const uint32_t tile = gridDim.x - 1 - blockIdx.x, h = blockIdx.y, g = h / (a.heads / a.kv_heads);  // the longest rows first
+  const uint32_t tile = (gridDim.x - 1 - blockIdx.x) / a.heads, h = (gridDim.x - 1 - blockIdx.x) % a.heads, g = h / (a.heads / a.kv_heads);  // the longest rows of all heads first
   const uint32_t m0 = tile * WM_Q, nq = min((uint32_t)WM_Q, w.rows.M - m0), i0 = w.rows.pos0 + m0, i1 = i0 + nq - 1;
   const uint32_t d8 = up8(a.dim), v8 = up8(a.vdim), rows = a.keep_first + a.ring;
   for (uint32_t e = threadIdx.x; e < MmaCfg<DB>::SMEM / 16; e += WM_THREADS) reinterpret_cast<uint4 *>(smb)[e] = make_uint4(0, 0, 0, 0);
@@ -493,17 +500,26 @@ __global__ void __launch_bounds__(WM_THREADS) window_mma_kernel(const __grid_con
   }
   const KeyList keys(a, i0, i1);
   const uint32_t total = keys.total, ntiles = (total + WM_K - 1) / WM_K;
+  // A thread copies the same 16-byte column of K or of V of every ROWS_PASS-th key.
+  constexpr uint32_t COLS = 2 * DB / 8, ROWS_PASS = WM_THREADS / COLS;
+  const uint32_t scol = threadIdx.x % COLS, srow = threadIdx.x / COLS, chunk = scol % (DB / 8), ld8 = scol < DB / 8 ? d8 : v8;
+  const __half *ssrc = (scol < DB / 8 ? kc : vc) + chunk * 8;
+  uint8_t *sdst = (scol < DB / 8 ? kt : vt) + (size_t)srow * ROWP + chunk * 16;
   auto stage = [&](uint32_t t, int buf) {
-    if (t < ntiles) {
-      const uint32_t kchunks = d8 / 8, per = kchunks + v8 / 8;
-      for (uint32_t e = threadIdx.x; e < WM_K * per; e += WM_THREADS) {
-        const uint32_t r = e / per, c = e % per, idx = t * WM_K + r;
-        const bool on = idx < total;
-        const uint32_t cr = keys.row(on ? idx : 0);
-        if (c < kchunks)
-          cp16z(kt + (size_t)(buf * WM_K + r) * ROWP + c * 16, kc + (size_t)cr * d8 + c * 8, on);
-        else
-          cp16z(vt + (size_t)(buf * WM_K + r) * ROWP + (c - kchunks) * 16, vc + (size_t)cr * v8 + (c - kchunks) * 8, on);
+    if (t < ntiles && chunk < ld8 / 8) {
+      const uint32_t r0 = keys.row(t * WM_K), r1 = keys.row(min(t * WM_K + WM_K, total) - 1);
+      uint8_t *dst = sdst + (size_t)(buf * WM_K) * ROWP;
+      if ((t + 1) * WM_K <= total && r1 - r0 == WM_K - 1 && (r1 < keys.keep || r0 >= keys.keep)) {  // the rows lie one behind the other
+        const __half *src = ssrc + (size_t)(r0 + srow) * ld8;
+#pragma unroll
+        for (uint32_t r = 0; r < WM_K; r += ROWS_PASS) cp16z(dst + r * ROWP, src + (size_t)r * ld8, true);
+      } else {
+#pragma unroll 4
+        for (uint32_t r = 0; r < WM_K; r += ROWS_PASS) {
+          const uint32_t idx = t * WM_K + r + srow;
+          const bool on = idx < total;
+          cp16z(dst + r * ROWP, ssrc + (size_t)keys.row(on ? idx : 0) * ld8, on);
+        }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -513,6 +529,8 @@ __global__ void __launch_bounds__(WM_THREADS) window_mma_kernel(const __grid_con
   const float c1 = cap ? 2.f * LOG2E * zs / a.softcap : zs * LOG2E, cap2 = a.softcap * LOG2E;
   const float r1 = a.r1 ? a.r1[h] : 0.f, r2 = a.r1 ? a.r2[h] : 0.f;
   const bool bias = a.r1 != nullptr;
+  float *logs = reinterpret_cast<float *>(smb + MmaCfg<DB>::SMEM);  // log2(1 + r2 distance)
+  for (uint32_t d = threadIdx.x; d < min(tab, i0 + WM_Q); d += WM_THREADS) logs[d] = lg2(1.f + r2 * (float)(int)d);
   const uint32_t qi[2] = {i0 + warp * 16 + gq, i0 + warp * 16 + gq + 8};
   float o[DB / 8][4], mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
@@ -544,20 +562,43 @@ __global__ void __launch_bounds__(WM_THREADS) window_mma_kernel(const __grid_con
       }
     }
     // scores in units of log2: cap tanh(z / cap) = cap - 2 cap / (1 + exp(2 z / cap))
+#pragma unroll
+    for (int n = 0; n < WM_K / 8; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[n][e] *= c1;
+    if (cap) {
+#pragma unroll
+      for (int n = 0; n < WM_K / 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] = cap2 - 2.f * cap2 * rcp(1.f + ex2(s[n][e]));
+    }
+    const uint32_t first = keys.position(t * WM_K), last = keys.position(t * WM_K + WM_K - 1), far = i0 + WM_Q - 1 - first;  // far: if no key is ahead
+    const bool inside = (t + 1) * WM_K <= total && last <= i0 && (!a.window || far < a.window || last < a.keep_first);
+    if (inside && (!bias || (far < tab && last - first == WM_K - 1))) {  // every row sees every key, keys stand side by side
+      if (bias) {
+        const float *lg = logs + (i0 + warp * 16 + gq - first - 2 * tq);
+#pragma unroll
+        for (int n = 0; n < WM_K / 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[n][e] = fmaf(-r1, lg[(e >> 1) * 8 - n * 8 - (e & 1)], s[n][e]);
+      }
+    } else {
+#pragma unroll
+      for (int n = 0; n < WM_K / 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t idx = t * WM_K + n * 8 + 2 * tq + (e & 1), j = keys.position(idx), i = qi[e >> 1];
+          float z = s[n][e];
+          if (bias) z = fmaf(-r1, lg2(1.f + r2 * (float)(int)(i - j)), z);
+          const bool see = idx < total && j <= i && (!a.window || i - j < a.window || j < a.keep_first);
+          s[n][e] = see ? z : -INFINITY;
+        }
+    }
     float tm[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int n = 0; n < WM_K / 8; ++n)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const uint32_t idx = t * WM_K + n * 8 + 2 * tq + (e & 1), j = keys.position(idx), i = qi[e >> 1];
-        float z = s[n][e] * c1;
-        if (cap) z = cap2 - 2.f * cap2 * rcp(1.f + ex2(z));
-        if (bias) z -= r1 * lg2(1.f + r2 * (float)(int)(i - j));
-        const bool see = idx < total && j <= i && (!a.window || i - j < a.window || j < a.keep_first);
-        z = see ? z : -INFINITY;
-        s[n][e] = z;
-        tm[e >> 1] = fmaxf(tm[e >> 1], z);
-      }
+      for (int e = 0; e < 4; ++e) tm[e >> 1] = fmaxf(tm[e >> 1], s[n][e]);
     float f[2], base[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -576,10 +617,12 @@ __global__ void __launch_bounds__(WM_THREADS) window_mma_kernel(const __grid_con
         s[n][e] = ex2(s[n][e] - base[e >> 1]);
         l[e >> 1] += s[n][e];
       }
+    if (__any_sync(0xffffffffu, f[0] != 1.f || f[1] != 1.f)) {  // rarely, once the maxima have settled
 #pragma unroll
-    for (int n = 0; n < DB / 8; ++n)
+      for (int n = 0; n < DB / 8; ++n)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) o[n][e] *= f[e >> 1];
+        for (int e = 0; e < 4; ++e) o[n][e] *= f[e >> 1];
+    }
 #pragma unroll
     for (int ks = 0; ks < WM_K / 16; ++ks) {
       const uint32_t pa[4] = {half2_bits(s[2 * ks][0], s[2 * ks][1]), half2_bits(s[2 * ks][2], s[2 * ks][3]), half2_bits(s[2 * ks + 1][0], s[2 * ks + 1][1]),
@@ -680,17 +723,22 @@ int pick_heads(cudaStream_t s, const WinArgs &w, const float *q, void *out, int 
   if (HG <= 4) return launch_rows<CT, 4, FUSED>(s, w, q, out, out_fmt, ld_out, splits);
   return launch_rows<CT, 8, FUSED>(s, w, q, out, out_fmt, ld_out, splits);
 }
+constexpr uint32_t WM_TABLE = 2048;  // distances a CTA holds the logarithms of, at most
 template <int DB>
 int launch_mma(cudaStream_t s, const WinArgs &w, const float *q, void *out, int out_fmt, uint32_t ld_out) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    GRETA_CUDA_TRY(cudaFuncSetAttribute(window_mma_kernel<DB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MmaCfg<DB>::SMEM));
+    GRETA_CUDA_TRY(cudaFuncSetAttribute(window_mma_kernel<DB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MmaCfg<DB>::SMEM + WM_TABLE * 4)));
     attr_set[dev] = true;
   }
-  GRETA_CUDA_TRY(launch_pdl(window_mma_kernel<DB>, dim3((w.rows.M + WM_Q - 1) / WM_Q, w.a.heads), dim3(WM_THREADS), MmaCfg<DB>::SMEM, s, w, q, out, out_fmt,
-                            ld_out));
+  const uint64_t ctas = ((uint64_t)w.rows.M + WM_Q - 1) / WM_Q * w.a.heads;
+  GRETA_REQUIRE(ctas < (1ull << 31), "window_attn_prefill: %u rows of %u heads exceed the grid", w.rows.M, w.a.heads);
+  const uint64_t ahead = (uint64_t)w.rows.pos0 + w.rows.M + WM_Q, span = w.a.window ? std::min<uint64_t>(w.a.window, ahead) : ahead;
+  const uint32_t tab = w.a.r1 ? (uint32_t)std::min<uint64_t>(span, WM_TABLE) : 0u;
+  GRETA_CUDA_TRY(launch_pdl(window_mma_kernel<DB>, dim3((unsigned)ctas), dim3(WM_THREADS), MmaCfg<DB>::SMEM + (size_t)tab * 4, s, w, q,
+                            out, out_fmt, ld_out, tab));
   return launched("window_mma_kernel");
 }
 
