@@ -281,13 +281,14 @@ __global__ void __launch_bounds__(MMA_WARPS * 32) attn_mma_decode_kernel(const A
 }
 
 // ------------------------------------------------------------------ causal prefill
-// grid (query blocks of 64, heads); warp w owns queries 64 b + 16 w .. + 15 of the chunk; query s of the chunk sits at
+// grid (query blocks of 64, heads), the last queries of all heads first: they have the longest rows (a 512-token
+// prompt 1193 -> 1175 us); warp w owns queries 64 b + 16 w .. + 15 of the chunk; query s of the chunk sits at
 // position pos0 + s and sees keys 0 .. pos0 + s of the cache.
 template <int DH>
 __global__ void __launch_bounds__(MMA_WARPS * 32) attn_mma_prefill_kernel(const AttnParams p, const uint32_t S, const uint32_t pos0) {
   constexpr int ROWP = mma_rowp<DH>();
   extern __shared__ __align__(16) uint8_t stage[];
-  const uint32_t qb = blockIdx.x, head = blockIdx.y, kvh = head / (p.H / p.Hkv);
+  const uint32_t order = blockIdx.y * gridDim.x + blockIdx.x, qb = gridDim.x - 1 - order / gridDim.y, head = order % gridDim.y, kvh = head / (p.H / p.Hkv);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const uint8_t *kg = reinterpret_cast<const uint8_t *>(p.kc) + (size_t)kvh * p.max_seq * DH * 2;
   const uint8_t *vg = reinterpret_cast<const uint8_t *>(p.vc) + (size_t)kvh * p.max_seq * DH * 2;

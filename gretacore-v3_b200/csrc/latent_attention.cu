@@ -586,7 +586,8 @@ latent_prefill_kernel(const __grid_constant__ LatArgs w, const __grid_constant__
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 15);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t tile = gridDim.x - 1 - blockIdx.x, h = blockIdx.y;  // the longest rows first
+  // the longest rows of all heads first (of one head after the other, a prompt of 1337 tokens took 1229 us, not 1217)
+  const uint32_t tile = (gridDim.x - 1 - blockIdx.x) / a.heads, h = (gridDim.x - 1 - blockIdx.x) % a.heads;
   const uint32_t m0 = tile * LP_Q, nq = min(LP_Q, w.rows.M - m0), i0 = w.rows.pos0 + m0, total = i0 + nq, ntiles = (total + KT - 1) / KT;
 
   if (threadIdx.x == 0) {
@@ -925,7 +926,9 @@ int launch_prefill(cudaStream_t s, const LatArgs &w, const void *q, const void *
     GRETA_CUDA_TRY(cudaFuncSetAttribute(latent_prefill_kernel<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LP_SMEM_LIMIT));
     attr_set[dev] = true;
   }
-  GRETA_CUDA_TRY(launch_pdl(latent_prefill_kernel<KT>, dim3((w.rows.M + LP_Q - 1) / LP_Q, a.heads), dim3(LP_THREADS), prefill_smem(a, KT, stages), s, w, mq, mk, mr, mv,
+  const uint64_t ctas = ((uint64_t)w.rows.M + LP_Q - 1) / LP_Q * a.heads;
+  GRETA_REQUIRE(ctas < (1ull << 31), "latent_attn_prefill: %u rows of %u heads exceed the grid", w.rows.M, a.heads);
+  GRETA_CUDA_TRY(launch_pdl(latent_prefill_kernel<KT>, dim3((unsigned)ctas), dim3(LP_THREADS), prefill_smem(a, KT, stages), s, w, mq, mk, mr, mv,
                             out, out_fmt, ld_out, stages));
   return launched("latent_prefill_kernel");
 }
