@@ -55,8 +55,19 @@ __global__ void __launch_bounds__(CL_WARPS * 32) attn_cluster_kernel(const AttnP
   __shared__ float res[Dh + 2];  // running maximum, normaliser, unnormalised output of this CTA's keys
   cg::cluster_group cluster = cg::this_cluster();
   pdl_launch_dependents();
-  pdl_wait();  // q, the position and the newest cache row come from the previous kernel
   const uint32_t split = cluster.block_rank(), head = blockIdx.y, qi = blockIdx.z;
+  if (sizeof(KV) == 2 && head % (p.H / p.Hkv) == 0) {  // this CTA's rows start their way from HBM to L2 while it still waits
+    // Only hints: neither the position nor the rows need be final yet.
+    const uint32_t L = min((p.d_pos ? __ldcg(p.d_pos + qi * p.pos_stride) : p.len0) + qi * p.len_step, p.max_seq), chunk = (L + CL_SPLITS - 1) / CL_SPLITS;
+    const uint32_t k0 = min(L, split * chunk), k1 = min(L, k0 + chunk);
+    const size_t at = ((size_t)qi * p.seq_stride + ((size_t)(head / (p.H / p.Hkv)) * p.max_seq + k0) * Dh) * 2;
+    const char *kp = reinterpret_cast<const char *>(p.kc) + at, *vp = reinterpret_cast<const char *>(p.vc) + at;
+    for (uint32_t b = threadIdx.x * 128; b < (k1 - k0) * Dh * 2; b += CL_WARPS * 32 * 128) {
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(kp + b));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(vp + b));
+    }
+  }
+  pdl_wait();  // q, the position and the newest cache row come from the previous kernel
   const uint32_t L = min((p.d_pos ? __ldcg(p.d_pos + qi * p.pos_stride) + 1 : p.len0) + qi * p.len_step, p.max_seq);  // never past the cache
   const uint32_t chunk = (L + CL_SPLITS - 1) / CL_SPLITS;
   const uint32_t k0 = split * chunk, k1 = min(L, k0 + chunk);
