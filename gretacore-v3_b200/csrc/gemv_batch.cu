@@ -942,6 +942,8 @@ size_t greta_cuda_gemv_batch_workspace_bytes(uint32_t M, uint32_t K) {
   return std::max(PREP_HEADER + (size_t)(K / 32) * mt * 1024, gemv_tc_workspace_bytes(M, K));
 }
 
+int greta_cuda_gemv_batch_route(int fmt, uint32_t M, uint64_t rows, uint32_t K) { return gemv_tc_route(fmt, M, rows, K); }
+
 int greta_cuda_gemv_batch(greta_stream_t stream, int fmt, const float *x, const float *gamma, float eps, const void *qs, const void *d,
                           const float *resid, float *y, uint32_t M, uint32_t N, uint32_t K, uint32_t k_slices, void *workspace) {
   if (N == 0) return GRETA_OK;

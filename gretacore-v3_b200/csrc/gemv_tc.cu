@@ -668,12 +668,16 @@ size_t gemv_tc_workspace_bytes(uint32_t M, uint32_t K) {
   return BT_HEADER + steps * tn * (BT_STEP * 4) + (size_t)BT_MAX_CTAS * 2 * 2 * tn * 128 * 4;
 }
 
+bool gemv_tc_route(int fmt, uint32_t M, uint64_t rows, uint32_t K) {
+  if (fmt != GRETA_FMT_Q4_0 && fmt != GRETA_FMT_Q8_0 && fmt != GRETA_FMT_F16) return false;
+  const uint64_t least = M > 8 || fmt == GRETA_FMT_Q8_0 ? BT_MIN_WEIGHTS : BT_MIN_WEIGHTS_FEW_ROWS;
+  return M >= 1 && M <= 32 && rows * K >= least && rows * K < (1ull << 40) && encode_tiled();
+}
+
 bool gemv_tc_takes(int fmt, int epi, const void *params) {
   const GemvParams &p = *static_cast<const GemvParams *>(params);
-  if (fmt != GRETA_FMT_Q4_0 && fmt != GRETA_FMT_Q8_0 && fmt != GRETA_FMT_F16) return false;
   const uint64_t rows = epi == EPI_SWIGLU ? (uint64_t)2 * p.N : (epi == EPI_QKV ? (uint64_t)(p.H + 2 * p.Hkv) * p.Dh : p.N);
-  const uint64_t least = p.M > 8 || fmt == GRETA_FMT_Q8_0 ? BT_MIN_WEIGHTS : BT_MIN_WEIGHTS_FEW_ROWS;
-  return rows * p.K >= least && rows * p.K < (1ull << 40) && (!p.gamma || aligned16(p.gamma)) && encode_tiled();
+  return gemv_tc_route(fmt, p.M, rows, p.K) && (!p.gamma || aligned16(p.gamma));
 }
 
 int gemv_tc(cudaStream_t stream, int fmt, int epi, const void *params, void *workspace) {

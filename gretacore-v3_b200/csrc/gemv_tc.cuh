@@ -12,6 +12,7 @@ constexpr uint64_t BT_MIN_WEIGHTS = 1ull << 20, BT_MIN_WEIGHTS_FEW_ROWS = 1ull <
 
 namespace greta {
 size_t gemv_tc_workspace_bytes(uint32_t M, uint32_t K);
+bool gemv_tc_route(int fmt, uint32_t M, uint64_t rows, uint32_t K);  // by formats and sizes alone
 // `params` is the GemvParams of the product (a type of its own in every file that includes gemv_device.cuh).
 bool gemv_tc_takes(int fmt, int epi, const void *params);
 int gemv_tc(cudaStream_t stream, int fmt, int epi, const void *params, void *workspace);

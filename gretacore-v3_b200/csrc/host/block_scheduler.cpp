@@ -56,7 +56,7 @@ TensorShard tensor_shard(const ModelConfig &c, LayerTensor t) {
 }
 
 namespace {
-constexpr size_t SKINNY_ROWS = 32;  // prompt rows up to which the projections are GEMVs on fp32 activations
+constexpr size_t SKINNY_ROWS = 32;  // prompt rows up to which the projections are the batched GEMVs on fp32 activations
 struct PlanePair {
   Buffer *qs, *d;
 };
@@ -167,15 +167,14 @@ bool BlockScheduler::allocate_activations(size_t batch_size, size_t max_seq_len,
   cur_seq_ = 0;
   if (c.arch == ModelArch::HYBRID) return allocate_hybrid_activations(err);
   const size_t S = std::max(max_seq_len, batch_size), D = c.dim, B = batch_size;
-  const size_t few = std::min<size_t>(S, SKINNY_ROWS);  // rows of what the route for more rows has no use for
   const size_t ql = (size_t)heads_l_ * c.head_dim, kvl = (size_t)kv_heads_l_ * c.head_dim;
   auto dev = [&](Buffer &b, size_t bytes, GretaDataType t = GretaDataType::FP32) { return b.allocate(bytes, BufferUsage::DeviceOnly, t, err); };
   ActivationBuffers &a = activations_;
   if (!dev(a.x, S * D * 4) || !dev(a.norm_out, S * D * 4) || !dev(a.q, S * ql * 4) || !dev(a.k, S * kvl * 4) || !dev(a.v, S * kvl * 4) ||
-      !dev(a.attn_out, S * ql * 4) || !dev(a.mlp_gate, S * hidden_l_ * 4) || !dev(a.mlp_up, few * hidden_l_ * 4) || !dev(a.mlp_out, (c.tp_size > 1 ? S : few) * D * 4))
+      !dev(a.attn_out, S * ql * 4) || !dev(a.mlp_gate, S * hidden_l_ * 4) || !dev(a.mlp_up, hidden_l_ * 4) || !dev(a.mlp_out, (c.tp_size > 1 ? S : 1) * D * 4))
     return false;
   if (S > SKINNY_ROWS && !dev(a.norm_f16, S * D * 2, GretaDataType::FP16)) return false;
-  if ((S > SKINNY_ROWS || B > 1) && !a.gave_up.allocate(16, BufferUsage::HostVisible, GretaDataType::FP32, err)) return false;
+  if (S > 1 && !a.gave_up.allocate(16, BufferUsage::HostVisible, GretaDataType::FP32, err)) return false;
   const size_t cache = (size_t)c.num_layers * B * kv_heads_l_ * max_seq_len * c.head_dim * 2;  // [L][B][Hkv][S][Dh] fp16
   if (!dev(a.kv_cache_k, cache, GretaDataType::FP16) || !dev(a.kv_cache_v, cache, GretaDataType::FP16)) return false;
   // d_pos: B positions, then B counts of ids produced; d_next: B token ids; out_tokens: [B][max_seq]
@@ -185,7 +184,8 @@ bool BlockScheduler::allocate_activations(size_t batch_size, size_t max_seq_len,
   if (!dev(a.attn_scratch, greta_cuda_attn_decode_scratch_bytes((uint32_t)B * heads_l_, c.head_dim))) return false;
   if (!dev(logits_, B * (size_t)c.vocab_size * 4)) return false;
   if (B > 1 && c.tp_size > 1 && !dev(logits_local_, B * (size_t)vocab_l_ * 4)) return false;
-  if (B > 1 && !dev(batch_ws_, greta_cuda_gemv_batch_workspace_bytes((uint32_t)B, std::max({c.dim, (uint32_t)ql, hidden_l_})))) return false;
+  const size_t rows = std::max(B, std::min(S, SKINNY_ROWS));  // of a batch, or of a short prompt
+  if (rows > 1 && !dev(batch_ws_, greta_cuda_gemv_batch_workspace_bytes((uint32_t)rows, std::max({c.dim, (uint32_t)ql, hidden_l_})))) return false;
   greta_cuda_memset(a.attn_scratch.data(), 0, a.attn_scratch.size(), nullptr);
   greta_cuda_memset(a.kv_cache_k.data(), 0, cache, nullptr);
   greta_cuda_memset(a.kv_cache_v.data(), 0, cache, nullptr);
@@ -584,9 +584,19 @@ bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t se
   return prompt_layer(layer_idx, seq_start, seq_len, true, err);
 }
 
+// Whether a product of a prompt of 2 to 32 rows goes to the kernel with bounded waits.
+bool BlockScheduler::short_prompt_waits(uint32_t S) const {
+  const ModelConfig &c = config_;
+  const int fmt = fmt_of(c.weight_type);
+  const uint64_t ql = (uint64_t)heads_l_ * c.head_dim, kvl = (uint64_t)kv_heads_l_ * c.head_dim;
+  return greta_cuda_gemv_batch_route(fmt, S, ql + 2 * kvl, c.dim) || greta_cuda_gemv_batch_route(fmt, S, c.dim, (uint32_t)ql) ||
+         greta_cuda_gemv_batch_route(fmt, S, 2 * (uint64_t)hidden_l_, c.dim) || greta_cuda_gemv_batch_route(fmt, S, c.dim, hidden_l_);
+}
+
 bool BlockScheduler::prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err) {
   // Prefill form of one layer over S = seq_len rows (the reference's operator order,
-  // block_scheduler.cpp:1814-3032): up to 32 rows by fp32 activations and the GEMVs, operator by operator, above on the tensor cores.
+  // block_scheduler.cpp:1814-3032): up to 32 rows by the batch's products on fp32 activations, a single one by the GEMVs, operator by
+  // operator, more than 32 by fp16 operands.
   const ModelConfig &c = config_;
   ActivationBuffers &a = activations_;
   if (layer_idx >= blocks_.size()) return fail(err, "execute_layer: layer out of range");
@@ -635,6 +645,29 @@ bool BlockScheduler::prompt_layer(size_t layer_idx, size_t seq_start, size_t seq
               "rmsnorm");
     GRETA_TRY(greta_cuda_gemm_segments(s, fmt, n16, S, D, ffn, 2, GRETA_GEMM_SWIGLU_F16), "w1, w3");
     return residual(gate16, b.w2, b.s_w2, hidden_l_, "w2");
+  }
+  // Up to 32 rows: norm, products that share their activations, SwiGLU and residual in one operator each, as for a batch (16 operators of their own and
+  // activations converted by every CTA before: 16 tokens through two layers of the 7B shape and its head took 518 us, now 328; 32 tokens 692 and 410).
+  if (S > 1) {
+    void *ws = batch_ws_.data();
+    auto residual = [&](const float *in, Buffer &w, Buffer &sw, uint32_t K, const char *name) -> bool {
+      GRETA_TRY(greta_cuda_gemv_batch(s, fmt, in, nullptr, 0.f, w.data(), sw.data(), tp ? nullptr : x, tp ? tmp : x, S, D, K, 0, ws), name);
+      if (!tp) return true;
+      if (all_reduce_(tmp, (size_t)S * D, s) != 0) return fail(err, "all-reduce failed");
+      GRETA_TRY(greta_cuda_add(s, x, tmp, x, (size_t)S * D), "residual");
+      return true;
+    };
+    const float *gamma = static_cast<const float *>(b.ffn_norm.data());
+    GRETA_TRY(greta_cuda_fused_rmsnorm_qkv_rope_kv_batch(s, fmt, x, static_cast<const float *>(b.attn_norm.data()), c.rms_eps, b.wq.data(), b.s_wq.data(), b.wk.data(),
+                                                         b.s_wk.data(), b.wv.data(), b.s_wv.data(), q, k, v, nullptr, nullptr, nullptr, S, heads_l_, kv_heads_l_, Dh,
+                                                         (uint32_t)max_seq_, c.rope_base, D, ws),
+              "qkv");
+    GRETA_TRY(greta_cuda_rope_kv(s, q, k, v, kc, vc, S, heads_l_, kv_heads_l_, Dh, c.rope_base, (uint32_t)seq_start, (uint32_t)max_seq_), "rope, kv update");
+    GRETA_TRY(greta_cuda_attn_prefill(s, q, kc, vc, att, S, (uint32_t)seq_start, heads_l_, kv_heads_l_, Dh, (uint32_t)max_seq_, scale), "attention");
+    if (!residual(att, b.wo, b.s_wo, ql, "wo")) return false;
+    if (keep_norm) GRETA_TRY(greta_cuda_rmsnorm(s, x, gamma, nrm, S, D, c.rms_eps), "rmsnorm");
+    GRETA_TRY(greta_cuda_fused_ffn_front_batch(s, fmt, x, gamma, c.rms_eps, b.w1.data(), b.s_w1.data(), b.w3.data(), b.s_w3.data(), gate, S, D, hidden_l_, ws), "w1, w3");
+    return residual(gate, b.w2, b.s_w2, hidden_l_, "w2");
   }
   auto proj = [&](const float *in, Buffer &w, Buffer &sw, float *out, uint32_t N, uint32_t K) -> int {
     return greta_cuda_gemv(s, fmt, in, 0, w.data(), sw.data(), out, S, N, K);
@@ -690,7 +723,8 @@ bool BlockScheduler::forward(const int32_t *tokens, size_t seq_start, size_t seq
       if (!prompt_layer(l, seq_start, seq_len, l + 1 == blocks_.size(), err)) return false;
   }
   if (!lm_head(static_cast<const float *>(a.x.data()) + (seq_len - 1) * c.dim, err)) return false;
-  int *gave_up = seq_len > SKINNY_ROWS ? static_cast<int *>(a.gave_up.data()) : nullptr;
+  const bool watched = seq_len > SKINNY_ROWS || (seq_len > 1 && short_prompt_waits((uint32_t)seq_len));
+  int *gave_up = watched ? static_cast<int *>(a.gave_up.data()) : nullptr;
   return products_finished(gave_up, "forward", "prompt", err);
 }
 

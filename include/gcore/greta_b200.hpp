@@ -645,6 +645,7 @@ private:
   bool lm_head_batch(std::string *err);
   bool step_fits(std::string *err) const;
   bool products_finished(int *gave_up, const char *what, const char *kind, std::string *err);
+  bool short_prompt_waits(uint32_t S) const;
   bool prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err);  // keep_norm: norm_out is filled
   void invalidate_graph();
   bool build_decode_plan(std::string *err);
@@ -684,7 +685,7 @@ private:
   bool graph_captured_ = false, initialized_ = false;
   size_t decode_steps_ = 0, decode_pos0_ = 0, max_seq_ = 0;
   uint32_t batch_ = 1, cur_seq_ = 0;      // sequences held; the one forward() / execute_layer() work on
-  gcore::rt::cuda::Buffer batch_ws_;      // batched decode: activations prepared for the tensor-core matmul kernels
+  gcore::rt::cuda::Buffer batch_ws_;      // batches and short prompts: workspace of the batched products
   gcore::rt::cuda::Buffer logits_local_;  // tensor-parallel batch: this rank's slice of the logits before placement
   AllReduceFn all_reduce_;
   greta_peer_exchange peer_{};            // tp == 0: not installed

@@ -241,6 +241,9 @@ GRETA_API size_t greta_cuda_gemv_batch_workspace_bytes(uint32_t M, uint32_t K);
 GRETA_API int greta_cuda_gemv_batch(greta_stream_t stream, int fmt, const float *x, const float *gamma, float eps,
                                     const void *qs, const void *d, const float *resid, float *y, uint32_t M, uint32_t N,
                                     uint32_t K, uint32_t k_slices, void *workspace);
+/* 1 where a product of M activation rows and `rows` x K weights (all that share the activations; workspace given, k_slices 0) goes through tcgen05, whose
+ * bounded waits report to greta_cuda_gemm_segments_status; 0 otherwise. */
+GRETA_API int greta_cuda_gemv_batch_route(int fmt, uint32_t M, uint64_t rows, uint32_t K);
 /* greta_cuda_fused_rmsnorm_qkv_rope_kv for M sequences: q_out [M][H*Dh]; row m is rotated at d_pos[m] and its K / V
  * go to row d_pos[m] of sequence m's cache; caches are fp16 [M][Hkv][max_seq][Dh]. */
 GRETA_API int greta_cuda_fused_rmsnorm_qkv_rope_kv_batch(

@@ -136,3 +136,34 @@ def test_a_batch_reports_a_product_that_gave_up(g):
         m.read_generated(1)
     assert np.asarray(m.read_generated(1)).shape == (2, 1)
     m.close()
+
+
+def _fmt(g, fmt):
+    return g.FMT_Q4_0 if fmt == "q4_0" else g.FMT_Q8_0
+
+
+@pytest.mark.parametrize("fmt", ["q4_0", "q8_0"])
+@pytest.mark.parametrize("n", [2, 9, 17, 32])
+def test_a_short_prompt_equals_its_tokens_one_by_one(g, fmt, n):
+    """Prompts of 2 to 32 tokens take the batched products (tcgen05 from 9 rows on with 4-bit weights, always with 8-bit ones); a token at a time takes the
+    single-row kernels.  Apart: fp32 sums in another order, then the fp16 cache of two layers.  A wait that gave up fails the prompt, once."""
+    pkg = load_package()
+    cfg = dict(dim=1024, num_heads=8, num_heads_kv=4, num_layers=2, vocab=1000, hidden_dim=2080, head_dim=128, max_seq=64, rope_base=1e4, rms_eps=1e-5)
+    m = pkg.model.Model(cfg, weight_fmt=_fmt(g, fmt))
+    m.load_synthetic(5)
+    prompt = pkg.model.synth_tokens(5, 40, cfg["vocab"])
+    for first in (0, 3):  # from the start of the sequence, and behind three tokens
+        if first:
+            m.forward(prompt[:first], 0)
+        whole = np.array(m.forward(prompt[first:first + n], first))
+        for i in range(first + n):
+            one = np.array(m.forward(prompt[i:i + 1], i))
+        assert np.linalg.norm(whole - one) < 2e-3 * np.linalg.norm(one)
+    waits = n > 8 or fmt == "q8_0"
+    assert bool(g.cuda().greta_cuda_gemv_batch_route(_fmt(g, fmt), n, 2 * cfg["hidden_dim"], cfg["dim"])) == waits
+    if waits:
+        g.check(g.cuda().greta_cuda_gemm_set_status(77))
+        with pytest.raises(RuntimeError, match="gave up.*77"):
+            m.forward(prompt[:n], 0)
+        m.forward(prompt[:n], 0)
+    m.close()
