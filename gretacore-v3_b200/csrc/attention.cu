@@ -56,8 +56,9 @@ __global__ void __launch_bounds__(CL_WARPS * 32) attn_cluster_kernel(const AttnP
   cg::cluster_group cluster = cg::this_cluster();
   pdl_launch_dependents();
   const uint32_t split = cluster.block_rank(), head = blockIdx.y, qi = blockIdx.z;
-  if (sizeof(KV) == 2 && head % (p.H / p.Hkv) == 0) {  // this CTA's rows start their way from HBM to L2 while it still waits
-    // Only hints: neither the position nor the rows need be final yet.
+  // This CTA's rows start their way from HBM to L2 while it still waits.  Only hints: neither the position nor the rows need be final yet.  Not over
+  // small caches, where it gains nothing (279 positions 486 -> 489 us for 8 steps; 520 positions 2021 -> 2000).
+  if (sizeof(KV) == 2 && p.max_seq >= 512 && head % (p.H / p.Hkv) == 0) {
     const uint32_t L = min((p.d_pos ? __ldcg(p.d_pos + qi * p.pos_stride) : p.len0) + qi * p.len_step, p.max_seq), chunk = (L + CL_SPLITS - 1) / CL_SPLITS;
     const uint32_t k0 = min(L, split * chunk), k1 = min(L, k0 + chunk);
     const size_t at = ((size_t)qi * p.seq_stride + ((size_t)(head / (p.H / p.Hkv)) * p.max_seq + k0) * Dh) * 2;

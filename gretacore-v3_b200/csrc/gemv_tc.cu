@@ -670,8 +670,8 @@ size_t gemv_tc_workspace_bytes(uint32_t M, uint32_t K) {
 
 bool gemv_tc_route(int fmt, uint32_t M, uint64_t rows, uint32_t K) {
   if (fmt != GRETA_FMT_Q4_0 && fmt != GRETA_FMT_Q8_0 && fmt != GRETA_FMT_F16) return false;
-  const uint64_t least = M > 8 || fmt == GRETA_FMT_Q8_0 ? BT_MIN_WEIGHTS : BT_MIN_WEIGHTS_FEW_ROWS;
-  return M >= 1 && M <= 32 && rows * K >= least && rows * K < (1ull << 40) && encode_tiled();
+  const uint64_t least = M <= 8 && fmt != GRETA_FMT_Q8_0 ? BT_MIN_WEIGHTS_FEW_ROWS : (K < BT_SHORT_K ? BT_MIN_WEIGHTS_SHORT : BT_MIN_WEIGHTS);
+  return M >= 1 && M <= 32 && K >= BT_STEP && rows * K >= least && rows * K < (1ull << 40) && encode_tiled();
 }
 
 bool gemv_tc_takes(int fmt, int epi, const void *params) {

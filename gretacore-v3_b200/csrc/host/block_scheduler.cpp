@@ -584,13 +584,20 @@ bool BlockScheduler::execute_layer(size_t layer_idx, size_t seq_start, size_t se
   return prompt_layer(layer_idx, seq_start, seq_len, true, err);
 }
 
-// Whether a product of a prompt of 2 to 32 rows goes to the kernel with bounded waits.
-bool BlockScheduler::short_prompt_waits(uint32_t S) const {
+// Whether a product of a layer goes to the kernel with bounded waits, for a prompt or a batch of 2 to 32 rows.
+bool BlockScheduler::layer_waits(uint32_t S) const {
   const ModelConfig &c = config_;
   const int fmt = fmt_of(c.weight_type);
   const uint64_t ql = (uint64_t)heads_l_ * c.head_dim, kvl = (uint64_t)kv_heads_l_ * c.head_dim;
   return greta_cuda_gemv_batch_route(fmt, S, ql + 2 * kvl, c.dim) || greta_cuda_gemv_batch_route(fmt, S, c.dim, (uint32_t)ql) ||
          greta_cuda_gemv_batch_route(fmt, S, 2 * (uint64_t)hidden_l_, c.dim) || greta_cuda_gemv_batch_route(fmt, S, c.dim, hidden_l_);
+}
+
+// Where a batch's step leaves the code of such a wait, or null where none of its products has any (asking costs a copy, 5 us).
+int *BlockScheduler::batch_gave_up() {
+  const bool waits = config_.arch != ModelArch::HYBRID && batch_ > 1 && batch_ <= SKINNY_ROWS &&
+                     (layer_waits((uint32_t)batch_) || greta_cuda_gemv_batch_route(fmt_of(config_.lm_head_type), (uint32_t)batch_, vocab_l_, config_.dim));
+  return waits ? static_cast<int *>(activations_.gave_up.data()) : nullptr;
 }
 
 bool BlockScheduler::prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err) {
@@ -723,7 +730,7 @@ bool BlockScheduler::forward(const int32_t *tokens, size_t seq_start, size_t seq
       if (!prompt_layer(l, seq_start, seq_len, l + 1 == blocks_.size(), err)) return false;
   }
   if (!lm_head(static_cast<const float *>(a.x.data()) + (seq_len - 1) * c.dim, err)) return false;
-  const bool watched = seq_len > SKINNY_ROWS || (seq_len > 1 && short_prompt_waits((uint32_t)seq_len));
+  const bool watched = seq_len > SKINNY_ROWS || (seq_len > 1 && layer_waits((uint32_t)seq_len));
   int *gave_up = watched ? static_cast<int *>(a.gave_up.data()) : nullptr;
   return products_finished(gave_up, "forward", "prompt", err);
 }
@@ -941,13 +948,13 @@ bool BlockScheduler::decode_step_host(const int32_t *token_in, int32_t *token_ou
   GRETA_TRY(greta_cuda_memcpy_h2d(activations_.d_next.data(), token_in, (size_t)batch_ * 4, s), "token upload");
   if (graph_->launch(stream_) != gcore::rt::GretaResult::SUCCESS) return fail(err, gcore::host::cuda_error("decode step launch failed"));
   GRETA_TRY(greta_cuda_memcpy_d2h(token_out, activations_.d_next.data(), (size_t)batch_ * 4, s), "token download");
-  if (!products_finished(batch_ > 1 ? static_cast<int *>(activations_.gave_up.data()) : nullptr, "decode_step_host", "batch", err)) return false;
+  if (!products_finished(batch_gave_up(), "decode_step_host", "batch", err)) return false;
   ++decode_steps_;
   return true;
 }
 
 bool BlockScheduler::read_generated(int32_t *out, size_t n, std::string *err) {
-  if (!products_finished(batch_ > 1 ? static_cast<int *>(activations_.gave_up.data()) : nullptr, "read_generated", "batch", err)) return false;
+  if (!products_finished(batch_gave_up(), "read_generated", "batch", err)) return false;
   if (n > decode_steps_) return fail(err, "read_generated: fewer steps were run");
   // out is [batch][n]; the device list is [batch][max_seq].  One strided copy: a copy per sequence cost 7 us each.
   return activations_.out_tokens.copy_rows_to_host(out, (size_t)max_seq_ * 4, n * 4, batch_, err);

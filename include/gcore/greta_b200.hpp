@@ -645,7 +645,8 @@ private:
   bool lm_head_batch(std::string *err);
   bool step_fits(std::string *err) const;
   bool products_finished(int *gave_up, const char *what, const char *kind, std::string *err);
-  bool short_prompt_waits(uint32_t S) const;
+  bool layer_waits(uint32_t S) const;
+  int *batch_gave_up();
   bool prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err);  // keep_norm: norm_out is filled
   void invalidate_graph();
   bool build_decode_plan(std::string *err);

@@ -50,7 +50,7 @@ def _out(g, n):
 
 
 @pytest.mark.parametrize("name", ["q4_0", "q8_0", "f16"])
-@pytest.mark.parametrize("M,N,K", [(9, 1100, 1056), (16, 130, 8256), (17, 4100, 544), (32, 2051, 2080), (32, 131, 33024), (2, 4700, 7232), (1, 4700, 7232)])
+@pytest.mark.parametrize("M,N,K", [(9, 1100, 1056), (16, 130, 8256), (17, 8100, 544), (32, 2051, 2080), (32, 131, 33024), (2, 4700, 7232), (1, 4700, 7232)])
 def test_products(g, name, M, N, K):
     lib, rng = g.cuda(), np.random.default_rng(M + N + K)
     w = _Weight(g, rng, name, N, K)
@@ -92,7 +92,7 @@ def test_gate_and_up(g, name, M, D, F):
 
 
 @pytest.mark.parametrize("name", ["q4_0", "q8_0"])
-@pytest.mark.parametrize("M,H,Hkv,Dh,D", [(17, 5, 1, 64, 4128), (9, 3, 3, 128, 1056), (32, 16, 2, 128, 512)])
+@pytest.mark.parametrize("M,H,Hkv,Dh,D", [(17, 5, 1, 64, 4128), (9, 3, 3, 128, 1056), (32, 16, 2, 128, 768)])
 def test_queries_keys_and_values(g, name, M, H, Hkv, Dh, D):
     """Segments that end inside a tile of 128 rows; rotation and cache rows at every sequence's own position, one of them past the cache."""
     lib, rng = g.cuda(), np.random.default_rng(M + H)
@@ -126,8 +126,8 @@ def test_queries_keys_and_values(g, name, M, H, Hkv, Dh, D):
 def test_a_batch_reports_a_product_that_gave_up(g):
     """The code of a bounded wait that gave up is written by the host here; reading the ids fails with it, once."""
     pkg = load_package()
-    cfg = dict(dim=256, num_heads=4, num_heads_kv=2, num_layers=1, vocab=500, hidden_dim=512, head_dim=64, max_seq=32, rope_base=1e4, rms_eps=1e-5)
-    m = pkg.model.Model(cfg, batch=2)
+    cfg = dict(dim=1024, num_heads=8, num_heads_kv=4, num_layers=1, vocab=500, hidden_dim=2080, head_dim=128, max_seq=32, rope_base=1e4, rms_eps=1e-5)
+    m = pkg.model.Model(cfg, weight_fmt=g.FMT_Q8_0, batch=2)
     m.load_synthetic(4)
     m.begin_decode(np.array([3, 4], np.int32), np.zeros(2, np.uint32))
     m.decode_step()
