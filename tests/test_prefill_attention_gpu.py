@@ -44,3 +44,32 @@ def test_prefill_attention_above_512_keys(g, S, pos0, H, Hkv, Dh, gain):
         want = (w / w.sum(1, keepdims=True)) @ v[h // (H // Hkv), :n].astype(np.float64)
         err = np.abs(got[:, h] - want).max() / want.std()
         assert err < 2e-5 * gain, err
+
+
+@pytest.mark.parametrize("S,pos0,H,Hkv,Dh,at", [(700, 0, 2, 1, 128, (5, 130, 255, 256, 640)), (300, 467, 2, 2, 64, (470, 511, 512, 766)), (40, 600, 4, 2, 128, (10, 605, 639)),
+                                                (130, 511, 1, 1, 64, (511, 512, 639, 640))])
+def test_values_that_are_no_finite_numbers_reach_no_earlier_row(g, S, pos0, H, Hkv, Dh, at):
+    """Infinities and NaNs in single columns of value rows `at`: rows in front of them are what they are with zeros there, up to the order of their
+    sums (tolerance as above); so are, to the bit, the columns without any; the rows that see them are no finite numbers in those columns."""
+    rng = np.random.default_rng(S + Dh)
+    n, ms = pos0 + S, pos0 + S + 3
+    q = rng.normal(0, 1, (S, H, Dh)).astype(np.float32)
+    k, v = (rng.normal(0, 1, (Hkv, ms, Dh)).astype(np.float16) for _ in range(2))
+    bad = np.zeros((Hkv, ms, Dh), bool)
+    for i, j in enumerate(at):
+        bad[i % Hkv, j, (7 * i) % Dh] = bad[Hkv - 1, j, Dh - 1 - i] = True
+    clean, dirty = v.copy(), v.copy()
+    clean[bad], dirty[bad] = 0, rng.choice(np.array([np.inf, -np.inf, np.nan], np.float16), int(bad.sum()))
+    out = []
+    for x in (clean, dirty):
+        dq, dk, dv = (g.DeviceBuffer.from_numpy(np.ascontiguousarray(a)) for a in (q, k.view(np.uint16), x.view(np.uint16)))
+        o = g.DeviceBuffer(S * H * Dh * 4)
+        g.check(g.cuda().greta_cuda_attn_prefill(None, dq.ptr, dk.ptr, dv.ptr, o.ptr, S, pos0, H, Hkv, Dh, ms, Dh ** -0.5))
+        g.check(g.cuda().greta_cuda_device_synchronize())
+        out.append(o.download(np.float32).reshape(S, H, Dh))
+    assert np.isfinite(out[0]).all()
+    sees = np.stack([np.stack([bad[h // (H // Hkv), :pos0 + i + 1].any(0) for h in range(H)]) for i in range(S)])  # [S][H][Dh]
+    assert not np.isfinite(out[1][sees]).any()
+    spared = ~bad.any(1)[np.arange(H) // (H // Hkv)]  # [H][Dh]
+    assert np.array_equal(out[1][:, spared], out[0][:, spared])
+    assert np.abs(out[1] - out[0])[~sees].max() < 2e-5 * out[0].std()
