@@ -48,7 +48,7 @@ struct AttnTcArgs {
 // one such token in the last tile take 13 ms instead of 0.1.  (Looking through the values in shared memory in front of the products took 0.2-0.5 us
 // per tile on the diagonal, 1-5 % of the kernel, whichever warp did it; a look at the outputs takes 0-1 %.)
 template <int DH>
-__device__ __noinline__ void sum_again(const AttnTcArgs &w, const uint8_t *qs, uint32_t h, uint32_t row, uint32_t i, uint32_t tiles_end, uint32_t c, float *y) {
+__device__ __noinline__ void sum_again(const AttnTcArgs &w, const uint8_t *qs, uint32_t h, uint32_t row, uint32_t i, uint32_t tiles_end, uint32_t c, bool halved, float *y) {
   const size_t at = (size_t)(h / w.group) * w.max_seq * DH;
   const __half *k = w.kc + at, *v = w.vc + at + c;
   const uint32_t end = min(tiles_end, w.pos0 + w.S);
@@ -77,7 +77,7 @@ __device__ __noinline__ void sum_again(const AttnTcArgs &w, const uint8_t *qs, u
         s[e] = fmaf(a.x + b.x, z.x, fmaf(a.y + b.y, z.y, s[e]));
       }
     }
-    const float t = (s[0] + s[1]) + (s[2] + s[3]), nm = fmaxf(mx, t), f = ex2(mx - nm), p = ex2(t - nm);
+    const float t = ((s[0] + s[1]) + (s[2] + s[3])) * (halved ? 2.f : 1.f), nm = fmaxf(mx, t), f = ex2(mx - nm), p = ex2(t - nm);
     mx = nm;
     l = fmaf(l, f, p);
 #pragma unroll
@@ -221,17 +221,26 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_prefill_kernel(const __
     const uint32_t quad = warp & 3, row = quad * 32 + lane, i = i0 + row;
     // ---- the warp's 32 queries, scaled, as pairs in the swizzled K-major layout
     constexpr uint32_t LPR = DH / 4, RPP = 32 / LPR;  // lanes per row, rows per pass
+    // Half the queries, and twice their scores, where one of them is past fp16 under log2(e): the range is that of q * scale, as in attention_mma.cu.
+    bool halved = false;
+    for (;;) {
+      const float by = halved ? 0.5f * w.scale2 : w.scale2;
+      float most = 0.f;
 #pragma unroll 8
-    for (uint32_t r0 = 0; r0 < 32; r0 += RPP) {
-      const uint32_t r = quad * 32 + r0 + lane / LPR, e = (lane % LPR) * 4;
-      float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < nq) f = *reinterpret_cast<const float4 *>(w.q + ((size_t)(m0 + r) * w.H + h) * DH + e);
-      f = make_float4(f.x * w.scale2, f.y * w.scale2, f.z * w.scale2, f.w * w.scale2);
-      const uint2 hi = make_uint2(half2_bits(f.x, f.y), half2_bits(f.z, f.w));
-      const float2 a = h2_to_f2(hi.x), b = h2_to_f2(hi.y);
-      uint8_t *dst = qs + (e / 64) * AT_SLAB + r * 128 + ((((e % 64) / 8) ^ (r & 7)) << 4) + (e & 4) * 2;
-      *reinterpret_cast<uint2 *>(dst) = hi;
-      *reinterpret_cast<uint2 *>(dst + SD * AT_SLAB) = make_uint2(half2_bits(f.x - a.x, f.y - a.y), half2_bits(f.z - b.x, f.w - b.y));
+      for (uint32_t r0 = 0; r0 < 32; r0 += RPP) {
+        const uint32_t r = quad * 32 + r0 + lane / LPR, e = (lane % LPR) * 4;
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < nq) f = *reinterpret_cast<const float4 *>(w.q + ((size_t)(m0 + r) * w.H + h) * DH + e);
+        f = make_float4(f.x * by, f.y * by, f.z * by, f.w * by);
+        most = fmaxf(most, fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))));
+        const uint2 hi = make_uint2(half2_bits(f.x, f.y), half2_bits(f.z, f.w));
+        const float2 a = h2_to_f2(hi.x), b = h2_to_f2(hi.y);
+        uint8_t *dst = qs + (e / 64) * AT_SLAB + r * 128 + ((((e % 64) / 8) ^ (r & 7)) << 4) + (e & 4) * 2;
+        *reinterpret_cast<uint2 *>(dst) = hi;
+        *reinterpret_cast<uint2 *>(dst + SD * AT_SLAB) = make_uint2(half2_bits(f.x - a.x, f.y - a.y), half2_bits(f.z - b.x, f.w - b.y));
+      }
+      if (halved || !__any_sync(0xffffffffu, most > 65504.f)) break;
+      halved = true;
     }
     fence_proxy_async();
     __syncwarp();
@@ -248,6 +257,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_prefill_kernel(const __
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld32(sb + c * 32, v[c]);
       tmem_ld_wait();
+      if (halved) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[c][j] = __float_as_uint(2.f * __uint_as_float(v[c][j]));
+      }
       if (t * AT_KEYS + AT_KEYS - 1 > i0) {  // the diagonal runs through the tile
 #pragma unroll
         for (int c = 0; c < 4; ++c)
@@ -328,7 +343,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_prefill_kernel(const __
           float y[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(o[j]);
-          sum_again<DH>(w, qs, h, row, i, ntiles * AT_KEYS, c, y);
+          sum_again<DH>(w, qs, h, row, i, ntiles * AT_KEYS, c, halved, y);
 #pragma unroll
           for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(y[j]);
         }

@@ -73,3 +73,22 @@ def test_values_that_are_no_finite_numbers_reach_no_earlier_row(g, S, pos0, H, H
     spared = ~bad.any(1)[np.arange(H) // (H // Hkv)]  # [H][Dh]
     assert np.array_equal(out[1][:, spared], out[0][:, spared])
     assert np.abs(out[1] - out[0])[~sees].max() < 2e-5 * out[0].std()
+
+
+@pytest.mark.parametrize("S,Dh,most", [(700, 128, 5.0e4), (530, 64, 6.5e4)])
+def test_queries_near_the_end_of_fp16(g, S, Dh, most):
+    """Queries whose largest |q * scale| is `most`, below 65504, against small keys.  Scores reach about 30: 22-bit queries leave weights 1e-5 open."""
+    rng = np.random.default_rng(S)
+    q, k = rng.normal(0, 1, (S, 1, Dh)).astype(np.float32), (rng.normal(0, 1, (S, Dh)) * 2.0 ** -14).astype(np.float16)
+    v, scale = rng.normal(0, 1, (S, Dh)).astype(np.float16), Dh ** -0.5
+    q = (q * (most / scale / np.abs(q).max())).astype(np.float32)
+    dq, dk, dv = (g.DeviceBuffer.from_numpy(a) for a in (q, k.view(np.uint16), v.view(np.uint16)))
+    o = g.DeviceBuffer(S * Dh * 4)
+    g.check(g.cuda().greta_cuda_attn_prefill(None, dq.ptr, dk.ptr, dv.ptr, o.ptr, S, 0, 1, 1, Dh, S, scale))
+    g.check(g.cuda().greta_cuda_device_synchronize())
+    s = q[:, 0].astype(np.float64) @ k.astype(np.float64).T * scale
+    assert 10 < np.abs(s).max() < 60
+    s[np.arange(S)[None] > np.arange(S)[:, None]] = -np.inf
+    w = np.exp(s - s.max(1, keepdims=True))
+    want = (w / w.sum(1, keepdims=True)) @ v.astype(np.float64)
+    assert np.abs(o.download(np.float32).reshape(S, Dh) - want).max() < 1e-4 * want.std()
