@@ -26,6 +26,7 @@ constexpr uint32_t AT_Q = 128, AT_KEYS = 128, AT_THREADS = 192, AT_TMEM = 512, A
 constexpr uint32_t AT_SLAB = 128 * 128;  // bytes of 64 columns of 128 rows
 constexpr float AT_LAZY = 8.f;           // a row's maximum may grow by this exponent before its sums are rescaled
 constexpr float AT_LOG2E = 1.4426950408889634f;
+constexpr float AT_LOWEST = -3.4028234e38f;  // a row's maximum before any score: scores of minus infinity have weight 0 whatever stands in front of them
 
 __device__ __forceinline__ void tma_load_3d(void *smem_dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(smem_dst)),
@@ -60,7 +61,7 @@ __device__ __noinline__ void sum_again(const AttnTcArgs &w, const uint8_t *qs, u
     if (j < end) hit |= 1u << e;
   }
   if (!hit) return;
-  float mx = -INFINITY, l = 0.f, acc[32];
+  float mx = AT_LOWEST, l = 0.f, acc[32];
 #pragma unroll
   for (int e = 0; e < 32; ++e) acc[e] = 0.f;
   for (uint32_t j = 0; j <= i && hit; ++j) {
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_prefill_kernel(const __
     __syncwarp();
     if (lane == 0) mbar_arrive(qf);
     const uint32_t lanes = tmem + (quad * 32 << 16);
-    float mx = -INFINITY, l = 0.f;
+    float mx = AT_LOWEST, l = 0.f;
     bool ok = true;
     for (uint32_t t = 0; t < ntiles && ok; ++t) {
       const uint32_t sb = lanes + (t & 1) * 128;
@@ -275,7 +276,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_prefill_kernel(const __
       for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int j = 0; j < 32; ++j) tm[j & 3] = fmaxf(tm[j & 3], __uint_as_float(v[c][j]));
-      const float nm = fmaxf(mx, fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])));  // finite from the first tile on: key 0
+      const float nm = fmaxf(mx, fmaxf(fmaxf(tm[0], tm[1]), fmaxf(tm[2], tm[3])));
       if (t == 0) {
         mx = nm;
       } else if (__any_sync(0xffffffffu, nm > mx + AT_LAZY)) {

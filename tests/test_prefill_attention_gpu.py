@@ -92,3 +92,21 @@ def test_queries_near_the_end_of_fp16(g, S, Dh, most):
     w = np.exp(s - s.max(1, keepdims=True))
     want = (w / w.sum(1, keepdims=True)) @ v.astype(np.float64)
     assert np.abs(o.download(np.float32).reshape(S, Dh) - want).max() < 1e-4 * want.std()
+
+
+def test_a_tile_of_scores_of_minus_infinity(g):
+    """The first 150 keys score minus infinity (both halves of the split query have the sign for it): rows behind them attend to the rest."""
+    S, Dh, rng = 600, 64, np.random.default_rng(1)
+    q, k, v = rng.normal(0, 1, (S, 1, Dh)).astype(np.float32), rng.normal(0, 1, (S, Dh)).astype(np.float16), rng.normal(0, 1, (S, Dh)).astype(np.float16)
+    scale = Dh ** -0.5
+    first = next(x for x in np.linspace(1, 2, 99, dtype=np.float32) if (f := np.float32(x * np.float32(np.float32(scale) * np.float32(1.4426950408889634)))) > np.float32(np.float16(f)))
+    q[:, 0, 0], k[:150, 0], k[150:, 0] = first, -np.inf, 0
+    dq, dk, dv = (g.DeviceBuffer.from_numpy(a) for a in (q, k.view(np.uint16), v.view(np.uint16)))
+    o = g.DeviceBuffer(S * Dh * 4)
+    g.check(g.cuda().greta_cuda_attn_prefill(None, dq.ptr, dk.ptr, dv.ptr, o.ptr, S, 0, 1, 1, Dh, S, scale))
+    g.check(g.cuda().greta_cuda_device_synchronize())
+    s = q[150:, 0].astype(np.float64) @ k[150:].astype(np.float64).T * scale
+    s[np.arange(S - 150)[None] > np.arange(S - 150)[:, None]] = -np.inf
+    w = np.exp(s - s.max(1, keepdims=True))
+    want = (w / w.sum(1, keepdims=True)) @ v[150:].astype(np.float64)
+    assert np.abs(o.download(np.float32).reshape(S, Dh)[150:] - want).max() < 2e-5 * want.std()
