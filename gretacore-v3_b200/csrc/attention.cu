@@ -508,6 +508,10 @@ int greta_cuda_attn_decode_static(greta_stream_t stream, const float *q, const v
                                   /*scratch_merge_only=*/true);
 }
 
+int greta_cuda_attn_prefill_route(uint32_t S, uint32_t pos0, uint32_t Dh) {
+  return tuning().attn_mma && S >= 8 && (Dh == 64 || Dh == 128) && (uint64_t)pos0 + S > 512;
+}
+
 static int attn_prefill_impl(greta_stream_t stream, const float *q, const void *kc, const void *vc, float *o, void *o16, uint32_t S, uint32_t pos0, uint32_t H,
                              uint32_t Hkv, uint32_t Dh, uint32_t max_seq, float scale) {
   if (S == 0) return GRETA_OK;
@@ -523,7 +527,7 @@ static int attn_prefill_impl(greta_stream_t stream, const float *q, const void *
     // tcgen05 above 512 keys: 1531 rows of 32 heads 98 against 256 us, 2048 rows of 64 heads of 64 168 against 365.  It would pay from 128 keys on (a
     // 512-token prompt of four 7B layers 1104 against 1190 us).  The line lies higher because the ids of the 512-token 7B run hang on a top-2
     // gap of 4.4e-6, less than what the products' sums leave open: with the smaller rounding error of this form one id of 128 is another.
-    if (pos0 + S > 512 && (!o16 || aligned16(o16)))
+    if (greta_cuda_attn_prefill_route(S, pos0, Dh) && (!o16 || aligned16(o16)))
       return attn_tc_prefill((cudaStream_t)stream, p, S, pos0, Dh, o16 ? o16 : (void *)o, o16 != nullptr);
     if (int rc = attn_mma_prefill((cudaStream_t)stream, p, S, pos0, Dh)) return rc;
   } else if (int rc = launch_attn<__half>((cudaStream_t)stream, p, S, Dh)) {

@@ -593,11 +593,9 @@ bool BlockScheduler::layer_waits(uint32_t S) const {
          greta_cuda_gemv_batch_route(fmt, S, 2 * (uint64_t)hidden_l_, c.dim) || greta_cuda_gemv_batch_route(fmt, S, c.dim, hidden_l_);
 }
 
-// Where a batch's step leaves the code of such a wait, or null where none of its products has any (asking costs a copy, 5 us).
-int *BlockScheduler::batch_gave_up() {
-  const bool waits = config_.arch != ModelArch::HYBRID && batch_ > 1 && batch_ <= SKINNY_ROWS &&
-                     (layer_waits((uint32_t)batch_) || greta_cuda_gemv_batch_route(fmt_of(config_.lm_head_type), (uint32_t)batch_, vocab_l_, config_.dim));
-  return waits ? static_cast<int *>(activations_.gave_up.data()) : nullptr;
+bool BlockScheduler::batch_waits() const {
+  return config_.arch != ModelArch::HYBRID && batch_ > 1 && batch_ <= SKINNY_ROWS &&
+         (layer_waits((uint32_t)batch_) || greta_cuda_gemv_batch_route(fmt_of(config_.lm_head_type), (uint32_t)batch_, vocab_l_, config_.dim));
 }
 
 bool BlockScheduler::prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err) {
@@ -621,6 +619,7 @@ bool BlockScheduler::prompt_layer(size_t layer_idx, size_t seq_start, size_t seq
   float *att = static_cast<float *>(a.attn_out.data()), *gate = static_cast<float *>(a.mlp_gate.data()), *up = static_cast<float *>(a.mlp_up.data());
   float *tmp = static_cast<float *>(a.mlp_out.data());
   const bool tp = c.tp_size > 1;
+  unasked_ = unasked_ || S > SKINNY_ROWS || (S > 1 && layer_waits(S)) || greta_cuda_attn_prefill_route(S, (uint32_t)seq_start, Dh);
   // More than 32 rows: products that share their activations in one launch, operands rounded to fp16 where they are made, SwiGLU and residual
   // in the products' epilogues.
   if (S > SKINNY_ROWS) {
@@ -730,22 +729,24 @@ bool BlockScheduler::forward(const int32_t *tokens, size_t seq_start, size_t seq
       if (!prompt_layer(l, seq_start, seq_len, l + 1 == blocks_.size(), err)) return false;
   }
   if (!lm_head(static_cast<const float *>(a.x.data()) + (seq_len - 1) * c.dim, err)) return false;
-  const bool watched = seq_len > SKINNY_ROWS || (seq_len > 1 && layer_waits((uint32_t)seq_len));
-  int *gave_up = watched ? static_cast<int *>(a.gave_up.data()) : nullptr;
-  return products_finished(gave_up, "forward", "prompt", err);
+  return finished("forward", err);
 }
 
-// Waits for the stream, and fails where a bounded wait of a tensor-core product gave up: results and cache rows are wrong then; the code is
-// reported once.  `gave_up` is page-locked, or null where the work had no such products.
-bool BlockScheduler::products_finished(int *gave_up, const char *what, const char *kind, std::string *err) {
+// Waits for the stream, and fails where a bounded wait gave up: results and cache rows are wrong then; the code is reported once.  Asking costs a copy (5 us),
+// so only what has such waits is asked.
+bool BlockScheduler::finished(const char *what, std::string *err) {
   cudaStream_t s = H(stream_);
+  int *gave_up = unasked_ ? static_cast<int *>(activations_.gave_up.data()) : nullptr;  // page-locked
   if (gave_up) GRETA_TRY(greta_cuda_gemm_segments_status(s, gave_up), what);
   GRETA_TRY(greta_cuda_stream_synchronize(s), what);
+  unasked_ = false;
   if (!gave_up || !*gave_up) return true;
   const int code = *gave_up;
   greta_cuda_gemm_set_status(0);
-  return fail(err, std::string(what) + ": a bounded wait of a " + kind + " product gave up (code " + std::to_string(code) + ")");
+  return fail(err, std::string(what) + ": a bounded wait of a tensor-core kernel gave up (code " + std::to_string(code) + ")");
 }
+
+bool BlockScheduler::finish(std::string *err) { return !unasked_ || finished("finish", err); }
 
 bool BlockScheduler::forward_logits(const int32_t *tokens, size_t seq_start, size_t seq_len, const uint32_t *rows, size_t n_rows, float *out,
                                     std::string *err) {
@@ -786,6 +787,7 @@ bool BlockScheduler::forward_logits(const int32_t *tokens, size_t seq_start, siz
 
 int32_t BlockScheduler::sample_greedy_gpu(size_t logits_offset_bytes, std::string *err) {
   int32_t id = -1;
+  if (!finish(err)) return id;
   gcore::rt::cuda::kernels::launch_argmax(H(stream_), static_cast<const float *>(logits_.data()) + logits_offset_bytes / 4, config_.vocab_size, &id);
   if (gcore::rt::cuda::kernels::last_launch_error() && err) *err = gcore::rt::cuda::kernels::last_launch_error_string();
   return id;
@@ -938,6 +940,7 @@ bool BlockScheduler::decode_step(std::string *err) {
   if (!step_fits(err)) return false;
   if (graph_->launch(stream_) != gcore::rt::GretaResult::SUCCESS) return fail(err, gcore::host::cuda_error("decode step launch failed"));
   ++decode_steps_;
+  unasked_ = unasked_ || batch_waits();
   return true;
 }
 
@@ -948,13 +951,14 @@ bool BlockScheduler::decode_step_host(const int32_t *token_in, int32_t *token_ou
   GRETA_TRY(greta_cuda_memcpy_h2d(activations_.d_next.data(), token_in, (size_t)batch_ * 4, s), "token upload");
   if (graph_->launch(stream_) != gcore::rt::GretaResult::SUCCESS) return fail(err, gcore::host::cuda_error("decode step launch failed"));
   GRETA_TRY(greta_cuda_memcpy_d2h(token_out, activations_.d_next.data(), (size_t)batch_ * 4, s), "token download");
-  if (!products_finished(batch_gave_up(), "decode_step_host", "batch", err)) return false;
+  unasked_ = unasked_ || batch_waits();
+  if (!finished("decode_step_host", err)) return false;
   ++decode_steps_;
   return true;
 }
 
 bool BlockScheduler::read_generated(int32_t *out, size_t n, std::string *err) {
-  if (!products_finished(batch_gave_up(), "read_generated", "batch", err)) return false;
+  if (!finished("read_generated", err)) return false;
   if (n > decode_steps_) return fail(err, "read_generated: fewer steps were run");
   // out is [batch][n]; the device list is [batch][max_seq].  One strided copy: a copy per sequence cost 7 us each.
   return activations_.out_tokens.copy_rows_to_host(out, (size_t)max_seq_ * 4, n * 4, batch_, err);

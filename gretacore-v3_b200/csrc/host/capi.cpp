@@ -220,11 +220,11 @@ int greta_model_forward_timed(greta_model_t m, const int32_t *tokens, uint32_t n
 }
 int greta_model_get_logits(greta_model_t m, float *out, uint32_t n) {
   std::string err;
-  return done(M(m)->sched.get_logits().copy_to_host(out, (size_t)n * 4, &err), err);
+  return done(M(m)->sched.finish(&err) && M(m)->sched.get_logits().copy_to_host(out, (size_t)n * 4, &err), err);
 }
 int greta_model_get_hidden(greta_model_t m, float *out, uint32_t row, uint32_t n) {
   std::string err;
-  return done(M(m)->sched.get_hidden_state().copy_to_host_offset(out, (size_t)row * M(m)->cfg.dim * 4, (size_t)n * 4, &err), err);
+  return done(M(m)->sched.finish(&err) && M(m)->sched.get_hidden_state().copy_to_host_offset(out, (size_t)row * M(m)->cfg.dim * 4, (size_t)n * 4, &err), err);
 }
 int greta_model_sample_greedy(greta_model_t m, int32_t *id) {
   std::string err;

@@ -550,7 +550,7 @@ struct BlockBuffers {
 
 struct ActivationBuffers {
   gcore::rt::cuda::Buffer x, q, k, v, attn_out, mlp_gate, mlp_up, mlp_out, norm_out;
-  gcore::rt::cuda::Buffer gave_up;                  // page-locked: code of a wait of the prompt's or the batch's products that gave up, 0 if none did
+  gcore::rt::cuda::Buffer gave_up;                  // page-locked: code of a wait of the prompt's or the batch's kernels that gave up, 0 if none did
   gcore::rt::cuda::Buffer norm_f16;                 // norm rows as the prompt's products read them
   gcore::rt::cuda::Buffer kv_cache_k, kv_cache_v;   // fp16 [L][Hkv_local][max_seq][Dh]
   gcore::rt::cuda::Buffer tokens, d_pos, d_next, attn_scratch, out_tokens;
@@ -601,6 +601,7 @@ public:
   bool set_layer_tensor_kquant(size_t layer, LayerTensor which, int ggml_type, const void *host, size_t bytes, std::string *err);
   bool set_global_tensor_kquant(GlobalTensor which, int ggml_type, const void *host, size_t bytes, std::string *err);
 
+  // Asynchronous, as decode_step(): before its rows are read through the buffers below, finish() says whether they are right.
   bool execute_layer(size_t layer_idx, size_t seq_start, size_t seq_len, const int32_t *tokens, std::string *err);
   // Runs seq_len tokens starting at seq_start; logits of the last position are left in get_logits().
   bool forward(const int32_t *tokens, size_t seq_start, size_t seq_len, std::string *err);
@@ -624,6 +625,9 @@ public:
   // Host-driven step: token id in from pinned host memory, sampled id out to pinned host memory, synchronised.
   bool decode_step_host(const int32_t *pinned_token_in, int32_t *pinned_token_out, std::string *err);
 
+  // Waits for the stream where execute_layer() or decode_step() launched kernels with bounded waits, and fails, once, where one of them gave up.
+  // forward(), read_generated(), decode_step_host() and sample_greedy_gpu() ask by themselves.
+  bool finish(std::string *err);
   gcore::rt::cuda::Buffer &get_hidden_state() { return activations_.x; }
   gcore::rt::cuda::Buffer &get_norm_out() { return activations_.norm_out; }  // fp32 rows of the last layer's feed-forward norm
   const gcore::rt::cuda::Buffer &get_logits() const { return logits_; }
@@ -644,9 +648,9 @@ private:
   bool decode_layers_batch(std::string *err);
   bool lm_head_batch(std::string *err);
   bool step_fits(std::string *err) const;
-  bool products_finished(int *gave_up, const char *what, const char *kind, std::string *err);
+  bool finished(const char *what, std::string *err);
   bool layer_waits(uint32_t S) const;
-  int *batch_gave_up();
+  bool batch_waits() const;
   bool prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err);  // keep_norm: norm_out is filled
   void invalidate_graph();
   bool build_decode_plan(std::string *err);
@@ -685,6 +689,7 @@ private:
   gcore::rt::GretaGraph *graph_ = nullptr;
   bool graph_captured_ = false, initialized_ = false;
   size_t decode_steps_ = 0, decode_pos0_ = 0, max_seq_ = 0;
+  bool unasked_ = false;                  // kernels with bounded waits were launched since their code was last asked for
   uint32_t batch_ = 1, cur_seq_ = 0;      // sequences held; the one forward() / execute_layer() work on
   gcore::rt::cuda::Buffer batch_ws_;      // batches and short prompts: workspace of the batched products
   gcore::rt::cuda::Buffer logits_local_;  // tensor-parallel batch: this rank's slice of the logits before placement

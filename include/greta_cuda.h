@@ -390,13 +390,16 @@ GRETA_API int greta_cuda_attn_decode_static(greta_stream_t stream, const float *
                                             uint32_t seq_len, uint32_t num_heads, uint32_t num_heads_kv,
                                             uint32_t head_dim, uint32_t max_seq_len, float scale);
 /* Causal prefill attention: q [S][H][Dh] fp32 against rows [pos0, pos0+S) of the
- * fp16 cache (keys 0 .. pos0+s for query s), o [S][H][Dh] fp32.
+ * fp16 cache (keys 0 .. pos0+s for query s), o [S][H][Dh] fp32.  Where greta_cuda_attn_prefill_route says 1 its waits are bounded, and one
+ * that gave up (rows of o are then not written) shows in greta_cuda_gemm_segments_status.
  * Replaces launch_flash_attention_prefill (attention_kernels.hip:543-618). */
 GRETA_API int greta_cuda_attn_prefill(greta_stream_t stream, const float *q, const void *k_cache_f16,
                                       const void *v_cache_f16, float *o, uint32_t S, uint32_t pos0,
                                       uint32_t num_heads, uint32_t num_heads_kv, uint32_t head_dim,
                                       uint32_t max_seq_len, float scale);
-/* The same, rounded to fp16; scratch: S * H * Dh floats, which some routes use. */
+/* 1 where S queries from position pos0 on go through tcgen05 (buffers 16-byte aligned), 0 otherwise. */
+GRETA_API int greta_cuda_attn_prefill_route(uint32_t S, uint32_t pos0, uint32_t head_dim);
+/* greta_cuda_attn_prefill rounded to fp16; scratch: S * H * Dh floats, which some routes use. */
 GRETA_API int greta_cuda_attn_prefill_f16(greta_stream_t stream, const float *q, const void *kc, const void *vc, void *o16, float *scratch, uint32_t S,
                                           uint32_t pos0, uint32_t H, uint32_t Hkv, uint32_t Dh, uint32_t max_seq, float scale);
 /* The reference's own prefill entry, launch_flash_attention_prefill (attention_kernels.hpp:124-128, kernel

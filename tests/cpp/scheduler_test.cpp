@@ -81,6 +81,24 @@ static int norm_out() {
   return 0;
 }
 
+// A bounded wait of a layer's kernels that gave up (its code is written by the host here) fails finish(), once; without such kernels nothing is asked.
+static int gave_up() {
+  ModelConfig c = small();
+  c.max_seq_len = 600;
+  BlockScheduler s;
+  if (!start(s, c)) return complain("start");
+  const std::vector<int32_t> t = prompt(600);
+  if (!s.forward(t.data(), 0, 520, &g_err)) return complain("forward");
+  const size_t portions[][2] = {{0, 40}, {520, 8}, {520, 32}};  // products with bounded waits; the attention alone
+  for (const auto &p : portions) {
+    if (!s.execute_layer(0, p[0], p[1], t.data(), &g_err) || greta_cuda_gemm_set_status(31) != GRETA_OK) return complain("execute_layer");
+    std::string err;
+    if (s.finish(&err) || err.find("31") == std::string::npos) return complain("finish passed, or hid the code: " + err);
+    if (!s.execute_layer(0, p[0], p[1], t.data(), &g_err) || !s.finish(&g_err)) return complain("the code was reported twice");
+  }
+  return s.execute_layer(0, 0, 8, t.data(), &g_err) && s.finish(&g_err) ? 0 : complain("few rows");
+}
+
 // Buffer::copy_rows_to_host: rows apart on the device, together on the host; nothing beyond the buffer's end.
 static int copy_rows() {
   gcore::rt::cuda::Buffer dev, pinned, none;
@@ -183,7 +201,7 @@ static int tensor_parallel() {
 
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
-  const int rc = what == "norm_out" ? norm_out() : what == "copy_rows" ? copy_rows() : what == "tensor_parallel" ? tensor_parallel() : 2;
+  const int rc = what == "norm_out" ? norm_out() : what == "copy_rows" ? copy_rows() : what == "gave_up" ? gave_up() : what == "tensor_parallel" ? tensor_parallel() : 2;
   printf("%s: %s\n", what.c_str(), rc ? "FAIL" : "PASS");
   return rc;
 }
