@@ -400,7 +400,7 @@ bool BlockScheduler::allocate_hybrid_activations(std::string *err) {
               !zeroed(w.decay, (size_t)R * w.decay_ld * 4) || !zeroed(w.o, (size_t)R * o * 4)))
     return false;
   if ((u && (!zeroed(w.u, (size_t)R * u * 4) || !zeroed(w.gate, (size_t)R * gate * 4))) || (q_latent && !zeroed(w.q_latent, (size_t)R * q_latent * cb)) ||
-      (scratch && !zeroed(w.latent_scratch, scratch)) || (scan && !zeroed(w.scan_scratch, scan)) || (kx && (!zeroed(w.q_tiles, qx, GretaDataType::FP16) || !zeroed(w.k_expanded, kx, GretaDataType::FP16) || !zeroed(w.v_expanded, vx, GretaDataType::FP16))))
+      (scratch && !zeroed(w.latent_scratch, scratch)) || (kx && (!zeroed(w.q_tiles, qx, GretaDataType::FP16) || !zeroed(w.k_expanded, kx, GretaDataType::FP16) || !zeroed(w.v_expanded, vx, GretaDataType::FP16))))
     return false;
   rotation_tables_ = std::vector<Buffer>(rotations_.size());
   for (size_t r = 0; r < rotations_.size(); ++r) {  // angles in double: the tables are as exact as their fp32 entries
@@ -437,6 +437,14 @@ bool BlockScheduler::allocate_hybrid_activations(std::string *err) {
     const GretaDataType ct = bf16 ? GretaDataType::FP16 : GretaDataType::FP32;
     if (!zeroed(b.k_cache, rows * up(m.dim, 8) * cb, ct) || !zeroed(b.v_cache, rows * up(m.vdim, 8) * cb, ct)) return false;
     if (m.taps && !zeroed(b.history, (size_t)B * m.taps * m.proj_cols() * 4)) return false;
+  }
+  // Scratch of the chunked scans (120 MB for 32 heads of 64): last, and only where as much again stays free for what is loaded afterwards.  Without it
+  // prompts take the scans token by token.
+  w.scan_scratch.free();
+  Buffer room;
+  if (scan && room.allocate(2 * scan, BufferUsage::DeviceOnly, GretaDataType::FP32, nullptr)) {
+    room.free();
+    w.scan_scratch.allocate(scan, BufferUsage::DeviceOnly, GretaDataType::FP32, nullptr);
   }
   GRETA_TRY(greta_cuda_device_synchronize(), "allocate_activations");
   invalidate_graph();

@@ -181,7 +181,10 @@ int greta_cuda_device_info(int device, char *name, size_t name_cap, int *sms, si
 int greta_cuda_malloc(void **ptr, size_t bytes) {
   GRETA_REQUIRE(ptr, "malloc: null out pointer");
   *ptr = nullptr;
-  GRETA_CUDA_TRY(cudaMalloc(ptr, bytes ? bytes : 1));
+  if (const cudaError_t e = cudaMalloc(ptr, bytes ? bytes : 1)) {
+    cudaGetLastError();  // reported here: the next launch has nothing to do with it
+    return cuda_fail(e, "cudaMalloc");
+  }
   return GRETA_OK;
 }
 int greta_cuda_free(void *ptr) {

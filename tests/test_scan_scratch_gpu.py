@@ -1,0 +1,38 @@
+"""A model whose chunked scans cannot have their scratch runs its prompts token by token."""
+import numpy as np
+import pytest
+
+from _support import load_package
+
+pytestmark = pytest.mark.gpu
+
+
+def test_a_model_that_fits_without_the_scratch():
+    import torch
+    pkg = load_package()
+    g = pkg.ffi
+    layer = {"type": "general_delta", "mlp": {"kind": "dense", "ff": 256}, "mixer": {"heads": 32, "dim": 128, "rank": 64}}
+    cfg = {"architecture": "Bidonex", "width": 512, "vocab": 1000, "max_positions": 1600, "norm": {"eps": 1e-6}, "layers": [layer]}
+    scratch = g.cuda().greta_cuda_delta_scan_scratch_bytes(32, 128, 1600)
+    assert scratch > 200 << 20
+    prompt = pkg.model.synth_tokens(3, 200, 1000)
+
+    def run():
+        m = pkg.model.Model.from_config(cfg)
+        free = torch.cuda.mem_get_info()[0]
+        m.load_synthetic(3)
+        before = g.cuda().greta_cuda_launch_count()
+        z = np.array(m.forward(prompt, 0))
+        launches = g.cuda().greta_cuda_launch_count() - before
+        m.close()
+        return z, launches, free
+
+    run()                                                      # whatever a first use loads
+    start = torch.cuda.mem_get_info()[0]
+    z, launches, free = run()
+    used = start - free                                        # by the model, scratch included
+    fill = g.DeviceBuffer(start - used + scratch // 2)
+    got, fewer, _ = run()
+    fill.free()
+    assert fewer < launches
+    assert np.linalg.norm(got - z) < 0.015 * np.linalg.norm(z)  # bf16 roundings behind sums in another order, as for whole models elsewhere
