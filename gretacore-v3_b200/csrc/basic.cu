@@ -6,6 +6,10 @@
 
 #include "greta_common.cuh"
 
+namespace greta {
+int gemm_ts_error_word(int **word);  // gemm_ts.cu
+}  // namespace greta
+
 using namespace greta;
 namespace cg = cooperative_groups;
 static inline cudaStream_t S(greta_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
@@ -199,7 +203,7 @@ __global__ void embedding_kernel(const int32_t *tokens, const void *__restrict__
 // of a 258 us step at 32000 logits; eight CTAs take 4 loads per thread, issued together, and meet through distributed shared memory.
 __global__ void __launch_bounds__(1024) argmax_kernel(const float *logits, uint32_t n,
                                                       int32_t *out, uint32_t *d_pos, int32_t *out_tokens,
-                                                      uint32_t *d_count, uint32_t out_capacity) {
+                                                      uint32_t *d_count, uint32_t out_capacity, const int *code) {
   __shared__ float sv[32];
   __shared__ uint32_t si[32];
   cg::cluster_group cluster = cg::this_cluster();
@@ -207,6 +211,7 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *logits, uint3
   pdl_wait();
   const uint32_t b = blockIdx.y, rank = blockIdx.x, ctas = gridDim.x;  // sequence: its own logits row, result, position, counter and output list
   logits += (size_t)b * n;
+  if (code && b == 0 && rank == 0 && threadIdx.x == 0) out[gridDim.y] = __ldcg(code);
   out += b;
   if (d_pos) d_pos += b;
   if (d_count) d_count += b;
@@ -278,10 +283,10 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *logits, uint3
 
 // Rows that one CTA covers with 4 loads per thread stay with it: a cluster's two barriers cost more than they save there.
 int launch_argmax(cudaStream_t stream, const float *logits, uint32_t n, uint32_t batch, int32_t *d_out, uint32_t *d_pos, int32_t *out_tokens,
-                  uint32_t *d_count, uint32_t out_capacity) {
+                  uint32_t *d_count, uint32_t out_capacity, const int *code = nullptr) {
   const unsigned ctas = n <= 4096 ? 1 : (n <= 8192 ? 2 : (n <= 16384 ? 4 : 8));
   GRETA_CUDA_TRY(launch_pdl_cluster(argmax_kernel, dim3(ctas, batch), dim3(1024), ctas, 0, stream, logits, n, d_out, d_pos, out_tokens, d_count,
-                                    out_capacity));
+                                    out_capacity, code));
   return launched("argmax_kernel");
 }
 
@@ -413,6 +418,14 @@ int greta_cuda_argmax_advance_batch(greta_stream_t stream, const float *logits, 
   GRETA_REQUIRE(n > 0 && batch >= 1 && batch <= 65535, "argmax_advance_batch: n=%u, batch=%u", n, batch);
   GRETA_REQUIRE(logits && d_next, "argmax_advance_batch: null pointer");
   return launch_argmax(S(stream), logits, n, batch, d_next, d_pos, d_out_tokens, d_count, out_capacity);
+}
+int greta_cuda_argmax_advance_batch_status(greta_stream_t stream, const float *logits, uint32_t n, uint32_t batch, int32_t *d_next, uint32_t *d_pos,
+                                           int32_t *d_out_tokens, uint32_t *d_count, uint32_t out_capacity) {
+  GRETA_REQUIRE(n > 0 && batch >= 1 && batch <= 65535, "argmax_advance_batch_status: n=%u, batch=%u", n, batch);
+  GRETA_REQUIRE(logits && d_next, "argmax_advance_batch_status: null pointer");
+  int *code = nullptr;
+  if (int rc = gemm_ts_error_word(&code)) return rc;
+  return launch_argmax(S(stream), logits, n, batch, d_next, d_pos, d_out_tokens, d_count, out_capacity, code);
 }
 int greta_cuda_silu(greta_stream_t stream, const float *x, float *y, size_t n) {
   if (n == 0) return GRETA_OK;

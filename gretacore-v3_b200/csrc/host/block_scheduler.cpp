@@ -174,11 +174,11 @@ bool BlockScheduler::allocate_activations(size_t batch_size, size_t max_seq_len,
       !dev(a.attn_out, S * ql * 4) || !dev(a.mlp_gate, S * hidden_l_ * 4) || !dev(a.mlp_up, hidden_l_ * 4) || !dev(a.mlp_out, (c.tp_size > 1 ? S : 1) * D * 4))
     return false;
   if (S > SKINNY_ROWS && !dev(a.norm_f16, S * D * 2, GretaDataType::FP16)) return false;
-  if (S > 1 && !a.gave_up.allocate(16, BufferUsage::HostVisible, GretaDataType::FP32, err)) return false;
+  if (S > 1 && !a.gave_up.allocate((B + 1) * 4, BufferUsage::HostVisible, GretaDataType::FP32, err)) return false;
   const size_t cache = (size_t)c.num_layers * B * kv_heads_l_ * max_seq_len * c.head_dim * 2;  // [L][B][Hkv][S][Dh] fp16
   if (!dev(a.kv_cache_k, cache, GretaDataType::FP16) || !dev(a.kv_cache_v, cache, GretaDataType::FP16)) return false;
-  // d_pos: B positions, then B counts of ids produced; d_next: B token ids; out_tokens: [B][max_seq]
-  if (!dev(a.tokens, S * 4) || !dev(a.d_pos, std::max<size_t>(16, 2 * B * 4)) || !dev(a.d_next, std::max<size_t>(16, B * 4)) ||
+  // d_pos: B positions, then B counts of ids produced; d_next: B token ids, then the code of a wait that gave up; out_tokens: [B][max_seq]
+  if (!dev(a.tokens, S * 4) || !dev(a.d_pos, std::max<size_t>(16, 2 * B * 4)) || !dev(a.d_next, std::max<size_t>(16, (B + 1) * 4)) ||
       !dev(a.out_tokens, B * max_seq_len * 4))
     return false;
   if (!dev(a.attn_scratch, greta_cuda_attn_decode_scratch_bytes((uint32_t)B * heads_l_, c.head_dim))) return false;
@@ -732,7 +732,7 @@ bool BlockScheduler::forward(const int32_t *tokens, size_t seq_start, size_t seq
   return finished("forward", err);
 }
 
-// Waits for the stream, and fails where a bounded wait gave up: results and cache rows are wrong then; the code is reported once.  Asking costs a copy (5 us),
+// Waits for the stream, and fails where a bounded wait gave up: results and cache rows are wrong then; the code is reported once.  Asking costs a copy (3 us),
 // so only what has such waits is asked.
 bool BlockScheduler::finished(const char *what, std::string *err) {
   cudaStream_t s = H(stream_);
@@ -740,8 +740,11 @@ bool BlockScheduler::finished(const char *what, std::string *err) {
   if (gave_up) GRETA_TRY(greta_cuda_gemm_segments_status(s, gave_up), what);
   GRETA_TRY(greta_cuda_stream_synchronize(s), what);
   unasked_ = false;
-  if (!gave_up || !*gave_up) return true;
-  const int code = *gave_up;
+  return !gave_up || no_wait_gave_up(*gave_up, what, err);
+}
+
+bool BlockScheduler::no_wait_gave_up(int code, const char *what, std::string *err) {
+  if (!code) return true;
   greta_cuda_gemm_set_status(0);
   return fail(err, std::string(what) + ": a bounded wait of a tensor-core kernel gave up (code " + std::to_string(code) + ")");
 }
@@ -901,9 +904,9 @@ bool BlockScheduler::begin_decode_batch(const int32_t *first_tokens, const uint3
       if (ok && c.tp_size > 1) ok = greta_cuda_memset(logits_.data(), 0, logits_.size(), s) == GRETA_OK;
       ok = ok && decode_layers_batch(err) && lm_head_batch(err);
       uint32_t *dp = static_cast<uint32_t *>(a.d_pos.data());
-      ok = ok && greta_cuda_argmax_advance_batch(s, static_cast<const float *>(logits_.data()), c.vocab_size, batch_,
-                                                 static_cast<int32_t *>(a.d_next.data()), dp, static_cast<int32_t *>(a.out_tokens.data()), dp + batch_,
-                                                 (uint32_t)max_seq_) == GRETA_OK;
+      ok = ok && (batch_waits() ? greta_cuda_argmax_advance_batch_status : greta_cuda_argmax_advance_batch)(
+                     s, static_cast<const float *>(logits_.data()), c.vocab_size, batch_, static_cast<int32_t *>(a.d_next.data()), dp,
+                     static_cast<int32_t *>(a.out_tokens.data()), dp + batch_, (uint32_t)max_seq_) == GRETA_OK;
     } else if (persistent_step_) {
       ok = greta_cuda_decode_layers(s, &desc, decode_plan_.data()) == GRETA_OK;
       if (!ok && err) *err = gcore::host::cuda_error("decode_layers");
@@ -950,9 +953,17 @@ bool BlockScheduler::decode_step_host(const int32_t *token_in, int32_t *token_ou
   cudaStream_t s = H(stream_);
   GRETA_TRY(greta_cuda_memcpy_h2d(activations_.d_next.data(), token_in, (size_t)batch_ * 4, s), "token upload");
   if (graph_->launch(stream_) != gcore::rt::GretaResult::SUCCESS) return fail(err, gcore::host::cuda_error("decode step launch failed"));
-  GRETA_TRY(greta_cuda_memcpy_d2h(token_out, activations_.d_next.data(), (size_t)batch_ * 4, s), "token download");
-  unasked_ = unasked_ || batch_waits();
-  if (!finished("decode_step_host", err)) return false;
+  if (batch_waits()) {  // the code comes behind the ids: a copy of its own took 3 us
+    int32_t *got = static_cast<int32_t *>(activations_.gave_up.data());
+    GRETA_TRY(greta_cuda_memcpy_d2h(got, activations_.d_next.data(), (size_t)(batch_ + 1) * 4, s), "token download");
+    GRETA_TRY(greta_cuda_stream_synchronize(s), "decode_step_host");
+    unasked_ = false;
+    if (!no_wait_gave_up(got[batch_], "decode_step_host", err)) return false;
+    std::copy(got, got + batch_, token_out);
+  } else {
+    GRETA_TRY(greta_cuda_memcpy_d2h(token_out, activations_.d_next.data(), (size_t)batch_ * 4, s), "token download");
+    if (!finished("decode_step_host", err)) return false;
+  }
   ++decode_steps_;
   return true;
 }

@@ -550,7 +550,7 @@ struct BlockBuffers {
 
 struct ActivationBuffers {
   gcore::rt::cuda::Buffer x, q, k, v, attn_out, mlp_gate, mlp_up, mlp_out, norm_out;
-  gcore::rt::cuda::Buffer gave_up;                  // page-locked: code of a wait of the prompt's or the batch's kernels that gave up, 0 if none did
+  gcore::rt::cuda::Buffer gave_up;                  // page-locked: code of a wait of the prompt's or the batch's kernels that gave up, 0 if none did; a host-driven batch's ids, then that code
   gcore::rt::cuda::Buffer norm_f16;                 // norm rows as the prompt's products read them
   gcore::rt::cuda::Buffer kv_cache_k, kv_cache_v;   // fp16 [L][Hkv_local][max_seq][Dh]
   gcore::rt::cuda::Buffer tokens, d_pos, d_next, attn_scratch, out_tokens;
@@ -649,6 +649,7 @@ private:
   bool lm_head_batch(std::string *err);
   bool step_fits(std::string *err) const;
   bool finished(const char *what, std::string *err);
+  bool no_wait_gave_up(int code, const char *what, std::string *err);
   bool layer_waits(uint32_t S) const;
   bool batch_waits() const;
   bool prompt_layer(size_t layer_idx, size_t seq_start, size_t seq_len, bool keep_norm, std::string *err);  // keep_norm: norm_out is filled

@@ -464,6 +464,10 @@ GRETA_API int greta_cuda_argmax_advance(greta_stream_t stream, const float *logi
 GRETA_API int greta_cuda_argmax_advance_batch(greta_stream_t stream, const float *logits, uint32_t n, uint32_t batch,
                                               int32_t *d_next, uint32_t *d_pos, int32_t *d_out_tokens, uint32_t *d_count,
                                               uint32_t out_capacity);
+/* The same, and d_next[batch] receives the code of greta_cuda_gemm_segments_status: one copy brings ids and code to the host. */
+GRETA_API int greta_cuda_argmax_advance_batch_status(greta_stream_t stream, const float *logits, uint32_t n, uint32_t batch,
+                                                     int32_t *d_next, uint32_t *d_pos, int32_t *d_out_tokens, uint32_t *d_count,
+                                                     uint32_t out_capacity);
 
 /* ------------------------------------------------------------------ dense linears (bf16 / fp32 weights)
  * Operators of the hybrid decoder designs (parallel attention / recurrent mixers over unquantised weights).  The reference

@@ -59,3 +59,21 @@ def test_what_a_batch_leaves_is_asked_for(read):
     assert ask() != 0 and b"gave up" in m.h.greta_host_last_error()
     assert ask() == 0
     m.close()
+
+
+def test_a_host_driven_batch_brings_the_code_with_its_ids():
+    pkg = load_package()
+    g, cfg = pkg.ffi, _cfg(dim=1024, num_heads=16, hidden_dim=2080, max_seq=32)
+    m = pkg.model.Model(cfg, weight_fmt=g.FMT_Q8_0, batch=5)
+    m.load_synthetic(4)
+    first, pos = np.arange(5, dtype=np.int32), np.zeros(5, np.uint32)
+    ids, _ = m.decode_e2e(first, pos, 6)
+    m.begin_decode(first, pos)
+    for _ in range(6):
+        m.decode_step()
+    assert np.array_equal(ids, m.read_generated(6))
+    g.check(g.cuda().greta_cuda_gemm_set_status(88))
+    with pytest.raises(RuntimeError, match="gave up.*88"):
+        m.decode_e2e(first, pos, 1)
+    assert np.array_equal(m.decode_e2e(first, pos, 6)[0], ids)
+    m.close()
