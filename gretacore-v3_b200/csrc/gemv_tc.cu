@@ -8,8 +8,8 @@
 // Small terms come first in the tensor core, which cuts every sum off at its last bit.  Error against 64 bits, 2-norm of the worst row, 16 rows:
 // 8192 x 8192 q4_0 1.3e-7 (mma.sync 2.2e-7), 4096 x 4096 fp16 1.5e-7 (1.6e-7).
 //
-// Measured in a CUDA graph with weights from HBM, both kernels of a product, us (mma.sync form behind the stroke): 16 rows q4_0 57344 x 8192 80 / 208
-// (3.3 TB/s), 8192 x 8192 23.5 / 34, 4096 x 4096 14.0 / 17.1; q8_0 101 / 245 (4.9 TB/s), 26 / 39, 14.3 / 20.0; fp16 155 / 284 (6.1 TB/s), 32 / 43, 16.2 / 16.3;
+// Measured in a CUDA graph with weights from HBM, both kernels of a product, us (mma.sync form behind the stroke): 16 rows q4_0 57344 x 8192 79 / 208
+// (3.3 TB/s), 8192 x 8192 20.8 / 34, 4096 x 4096 11.8 / 17.1; q8_0 101 / 245 (4.9 TB/s), 26 / 39, 14.3 / 20.0; fp16 155 / 284 (6.1 TB/s), 32 / 43, 16.2 / 16.3;
 // 32 rows q4_0 115 / 318, 30 / 51, 19.5 / 25.3.  What bounds q4_0: the chain load - unpack - store - multiply - read of a set of warps, of
 // which four run at a time; of 91 us alone at 57344 x 8192 the products left out give 77, reading and adding the sums 79, unpacking 93.
 //
@@ -21,7 +21,7 @@
 //                weights are multiplied out of shared memory as they came), its first warp issues the products, all scale and add the sums.
 // Two row tiles share an activation buffer: with one the activations from L2 are as many bytes as the weights from HBM.
 //
-// Work is cut into steps of 256 K x 256 rows, and every CTA takes an equal run of them (row tiles one after the other, K inside).  A row tile that
+// Work is cut into steps of 256 K x 256 rows, and every CTA takes a run of them (row tiles one after the other, K inside; plan_shares).  A row tile that
 // several CTAs share is summed through the workspace: each stores its part and takes a ticket; who comes last adds the parts in CTA order
 // (the result does not depend on who that was) and finishes the rows.  Nobody waits for another CTA.
 // Every wait is bounded, as in gemm_ts.cu; one that gave up is reported in the same word.
@@ -60,8 +60,9 @@ struct BtArgs {
   float *part;        // [CTA][2][2 tiles][TN][128]
   uint32_t *tickets;  // [CTA]
   uint32_t n[3], tile_end[3], tiles, steps;
-  uint32_t total;     // steps of all pairs of row tiles
   int *error;
+  // Runs of steps: column x of the grid's row y begins at step y * row + (x * run + min(x, longer)) * unit.
+  uint32_t row, run, longer, unit;
 };
 
 __device__ __forceinline__ void bulk_load(void *smem_dst, const void *src, uint32_t bytes, uint64_t *bar) {
@@ -87,9 +88,11 @@ __device__ __forceinline__ void int8_word(uint32_t w, uint32_t *o) {
   o[1] = hsub2_u(__byte_perm(t, 0x64646464u, 0x7362), C1152);
 }
 
-__device__ __forceinline__ uint32_t share_begin(uint32_t b, uint32_t total, uint32_t ctas) { return (uint32_t)((uint64_t)b * total / ctas); }
-// The CTA whose share holds step s.
-__device__ __forceinline__ uint32_t share_of(uint32_t s, uint32_t total, uint32_t ctas) { return (uint32_t)((((uint64_t)s + 1) * ctas - 1) / total); }
+// The CTA whose run holds step s, of runs in one row of the grid.
+__device__ __forceinline__ uint32_t run_of(const BtArgs &w, uint32_t s) {
+  const uint32_t u = s / w.unit, head = w.longer * (w.run + 1);
+  return u < head ? u / (w.run + 1) : w.longer + (u - head) / w.run;
+}
 
 struct TileAt {
   uint32_t seg, n0;
@@ -199,7 +202,8 @@ __global__ void __launch_bounds__(BT_THREADS, 1) gemv_tc_kernel(const __grid_con
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1), *last_flag = abort_flag + 1;
   float *factor = reinterpret_cast<float *>(tmem_slot + 4);  // [TN], then positions [TN]
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const uint32_t begin = share_begin(blockIdx.x, w.total, gridDim.x), end = share_begin(blockIdx.x + 1, w.total, gridDim.x);
+  const uint32_t cta = blockIdx.y * gridDim.x + blockIdx.x, begin = blockIdx.y * w.row + (blockIdx.x * w.run + min(blockIdx.x, w.longer)) * w.unit;
+  const uint32_t end = begin + (w.run + (blockIdx.x < w.longer ? 1 : 0)) * w.unit;
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < RAW; ++s) {
@@ -455,7 +459,7 @@ __global__ void __launch_bounds__(BT_THREADS, 1) gemv_tc_kernel(const __grid_con
       }
       const bool whole = count == w.steps;
       float *mine = buf + t * 16 * 128 + row;
-      float *part = w.part + ((size_t)(blockIdx.x * 2 + (k0 == 0 ? 1 : 0)) * 2 + t) * TN * 128 + row;
+      float *part = w.part + ((size_t)(cta * 2 + (k0 == 0 ? 1 : 0)) * 2 + t) * TN * 128 + row;
 #pragma unroll
       for (uint32_t g = 0; g < TN / 16; ++g) {
         if (h == 1) {
@@ -483,7 +487,8 @@ __global__ void __launch_bounds__(BT_THREADS, 1) gemv_tc_kernel(const __grid_con
         }
       }
       if (!whole) {
-        const uint32_t c0 = share_of(pair * w.steps, w.total, gridDim.x), c1 = share_of((pair + 1) * w.steps - 1, w.total, gridDim.x);
+        uint32_t c0 = blockIdx.y * gridDim.x, c1 = c0 + gridDim.x - 1;  // the CTAs that share the pair: a row of the grid, or out of the only one
+        if (w.row == 0) c0 = run_of(w, pair * w.steps), c1 = run_of(w, (pair + 1) * w.steps - 1);
         if (tid == 0) *last_flag = atomicAdd(w.tickets + c0, 1u) == c1 - c0;
         sync_workers();
         if (*last_flag) {
@@ -628,7 +633,7 @@ __global__ void __launch_bounds__(IMG_THREADS) prep_image_kernel(const float *x,
 }
 
 template <int FMT, int EPI, int TN>
-int launch_tc(cudaStream_t stream, const BtArgs &a, uint32_t ctas) {
+int launch_tc(cudaStream_t stream, const BtArgs &a, dim3 grid) {
   using P = BtPlan<FMT, TN>;
   static bool attr_set[64] = {};
   int dev = 0;
@@ -641,20 +646,20 @@ int launch_tc(cudaStream_t stream, const BtArgs &a, uint32_t ctas) {
   GRETA_CUDA_TRY(launch_pdl(prep_image_kernel<FMT>, dim3(TN), dim3(IMG_THREADS), 0, stream, static_cast<const float *>(p.x), p.gamma, p.eps, p.M, p.K, a.steps,
                             const_cast<float *>(a.rowmul), a.tickets, const_cast<uint8_t *>(a.image)));
   if (int rc = launched("prep_image_kernel")) return rc;
-  GRETA_CUDA_TRY(launch_pdl(gemv_tc_kernel<FMT, EPI, TN>, dim3(ctas), dim3(BT_THREADS), P::SMEM, stream, a));
+  GRETA_CUDA_TRY(launch_pdl(gemv_tc_kernel<FMT, EPI, TN>, grid, dim3(BT_THREADS), P::SMEM, stream, a));
   return launched("gemv_tc_kernel");
 }
 template <int FMT, int EPI>
-int launch_rows(cudaStream_t stream, const BtArgs &a, uint32_t ctas) {
-  return a.p.M <= 16 ? launch_tc<FMT, EPI, 16>(stream, a, ctas) : launch_tc<FMT, EPI, 32>(stream, a, ctas);
+int launch_rows(cudaStream_t stream, const BtArgs &a, dim3 grid) {
+  return a.p.M <= 16 ? launch_tc<FMT, EPI, 16>(stream, a, grid) : launch_tc<FMT, EPI, 32>(stream, a, grid);
 }
 template <int FMT>
-int launch_epi(cudaStream_t stream, int epi, const BtArgs &a, uint32_t ctas) {
+int launch_epi(cudaStream_t stream, int epi, const BtArgs &a, dim3 grid) {
   switch (epi) {
-    case EPI_PLAIN: return launch_rows<FMT, EPI_PLAIN>(stream, a, ctas);
-    case EPI_RESIDUAL: return launch_rows<FMT, EPI_RESIDUAL>(stream, a, ctas);
-    case EPI_SWIGLU: return launch_rows<FMT, EPI_SWIGLU>(stream, a, ctas);
-    default: return launch_rows<FMT, EPI_QKV>(stream, a, ctas);
+    case EPI_PLAIN: return launch_rows<FMT, EPI_PLAIN>(stream, a, grid);
+    case EPI_RESIDUAL: return launch_rows<FMT, EPI_RESIDUAL>(stream, a, grid);
+    case EPI_SWIGLU: return launch_rows<FMT, EPI_SWIGLU>(stream, a, grid);
+    default: return launch_rows<FMT, EPI_QKV>(stream, a, grid);
   }
 }
 
@@ -670,7 +675,9 @@ size_t gemv_tc_workspace_bytes(uint32_t M, uint32_t K) {
 
 bool gemv_tc_route(int fmt, uint32_t M, uint64_t rows, uint32_t K) {
   if (fmt != GRETA_FMT_Q4_0 && fmt != GRETA_FMT_Q8_0 && fmt != GRETA_FMT_F16) return false;
-  const uint64_t least = M <= 8 && fmt != GRETA_FMT_Q8_0 ? BT_MIN_WEIGHTS_FEW_ROWS : (K < BT_SHORT_K ? BT_MIN_WEIGHTS_SHORT : BT_MIN_WEIGHTS);
+  const bool few = M <= 16 && (fmt == GRETA_FMT_F16 || (fmt == GRETA_FMT_Q4_0 && K > 512));
+  const uint64_t least = M <= 8 && fmt != GRETA_FMT_Q8_0 ? BT_MIN_WEIGHTS_FEW_ROWS
+                                                         : (K < BT_SHORT_K ? (few ? BT_MIN_WEIGHTS_SHORT_FEW : BT_MIN_WEIGHTS_SHORT) : BT_MIN_WEIGHTS);
   return M >= 1 && M <= 32 && K >= BT_STEP && rows * K >= least && rows * K < (1ull << 40) && encode_tiled();
 }
 
@@ -678,6 +685,37 @@ bool gemv_tc_takes(int fmt, int epi, const void *params) {
   const GemvParams &p = *static_cast<const GemvParams *>(params);
   const uint64_t rows = epi == EPI_SWIGLU ? (uint64_t)2 * p.N : (epi == EPI_QKV ? (uint64_t)(p.H + 2 * p.Hkv) * p.Dh : p.N);
   return gemv_tc_route(fmt, p.M, rows, p.K) && (!p.gamma || aligned16(p.gamma));
+}
+
+// Into how many units of K steps a pair of row tiles is cut, every CTA taking an equal run of all units, and the CTAs.  Single steps in equal runs (parts = steps)
+// balance best, but a run that ends inside a pair leaves parts of two pairs to be summed through the workspace, each as long as three steps, and every part of a
+// pair costs its last CTA another read.  So also tried: every unit a CTA of its own, and whole pairs.  mma.sync form / equal runs only / as here, in a CUDA graph, us: 9 rows q4_0 23360 x 512 10.1 / 14.4 / 7.8, 5952 x 2048
+// 13.4 / 13.2 / 10.9, 1600 x 8192 16.4 / 16.2 / 13.3, 8192 x 8192 31.9 / 23.2 / 20.5; 8 rows q8_0 18624 x 640 11.6 / 13.7 / 9.4; 9 rows fp16 15552 x 768
+// 11.3 / 15.9 / 11.0; 32 rows q4_0 16384 x 4096 46.3 / 29.6 / 26.8.  Times in 10 ns, fitted to products of 16 to 3600 steps; a step of fp16 weights waits for its
+// 128 KB (38 bytes/ns and SM), and in long runs of those the first meeting is hidden.
+static uint32_t plan_shares(int fmt, uint32_t M, uint32_t steps, uint32_t pairs, uint32_t *ctas) {
+  const uint32_t most = std::min((uint32_t)sm_count(), BT_MAX_CTAS), all = steps * pairs;
+  const bool wide = M > 16, f16 = fmt == GRETA_FMT_F16;
+  const uint64_t step = f16 ? 330 : (fmt == GRETA_FMT_Q4_0 ? 160 : 205) + (wide ? 100 : 0);
+  const uint64_t meet = wide ? 660 : (f16 ? 650 : 430), part = wide ? 38 : 24, whole = wide ? 420 : (f16 ? 350 : 250);
+  *ctas = most;
+  // Long runs stay equal: there fewer CTAs cost the kernels around the product more than the meetings cost it (three parts of the pairs of 10240 x 8192, 16 rows: the
+  // product 27.6 -> 26.8, the layer it stands in 353 -> 367; up to 8 steps a CTA, layers of widths 1536 to 8192: 1-6 % faster).
+  if (all > 8 * most) return steps;
+  const uint32_t deal = (pairs + most - 1) / most;  // pairs of a CTA that takes whole ones
+  uint32_t parts = 1;
+  *ctas = std::min(most, pairs);
+  uint64_t best = (step * steps + whole) * deal;
+  for (uint32_t m = 2; m <= steps && m * pairs <= most; ++m) {
+    const uint64_t time = step * ((steps + m - 1) / m) + meet + part * m;
+    if (time < best) best = time, parts = m, *ctas = m * pairs;
+  }
+  if (all > most) {
+    const uint32_t run = (all + most - 1) / most, meetings = f16 && !wide && 2 * all > 5 * most ? 1 : 2;
+    const uint64_t time = step * all / most + meetings * (meet + part * std::min(steps, (steps + run - 1) / run + 1)) + (run > 2 * steps ? whole * (run / steps - 1) : 0);
+    if (time < best) parts = steps, *ctas = most;
+  }
+  return parts;
 }
 
 int gemv_tc(cudaStream_t stream, int fmt, int epi, const void *params, void *workspace) {
@@ -709,10 +747,19 @@ int gemv_tc(cudaStream_t stream, int fmt, int epi, const void *params, void *wor
   w.tickets = reinterpret_cast<uint32_t *>(ws + 256);
   w.image = ws + BT_HEADER;
   w.part = reinterpret_cast<float *>(ws + BT_HEADER + (size_t)w.steps * tn * (BT_STEP * 4));
-  w.total = (w.tiles + 1) / 2 * w.steps;
+  const uint32_t pairs = (w.tiles + 1) / 2;
+  uint32_t ctas;
+  const uint32_t parts = plan_shares(fmt, p.M, w.steps, pairs, &ctas);
+  dim3 grid(ctas);
+  if (parts > 1 && parts * pairs == ctas) {  // a unit each: a row of the grid per pair
+    grid = dim3(parts, pairs);
+    w.row = w.steps, w.run = w.steps / parts, w.longer = w.steps % parts, w.unit = 1;
+  } else {
+    const uint32_t units = parts * pairs;
+    w.row = 0, w.run = units / ctas, w.longer = units % ctas, w.unit = parts == 1 ? w.steps : 1;
+  }
   if (int rc = gemm_ts_error_word(&w.error)) return rc;
-  const uint32_t ctas = std::min({(uint32_t)sm_count(), BT_MAX_CTAS, w.total});
-  if (fmt == GRETA_FMT_F16) return launch_epi<GRETA_FMT_F16>(stream, epi, w, ctas);
-  return fmt == GRETA_FMT_Q4_0 ? launch_epi<GRETA_FMT_Q4_0>(stream, epi, w, ctas) : launch_epi<GRETA_FMT_Q8_0>(stream, epi, w, ctas);
+  if (fmt == GRETA_FMT_F16) return launch_epi<GRETA_FMT_F16>(stream, epi, w, grid);
+  return fmt == GRETA_FMT_Q4_0 ? launch_epi<GRETA_FMT_Q4_0>(stream, epi, w, grid) : launch_epi<GRETA_FMT_Q8_0>(stream, epi, w, grid);
 }
 }  // namespace greta

@@ -4,12 +4,13 @@
 
 constexpr uint32_t BT_MAX_CTAS = 160;
 constexpr size_t BT_HEADER = 1024;  // row factors, then tickets
-// Smallest products (weights) that go through tcgen05; below, launch and the meeting of CTAs cost more than gemv_batch.cu takes.  In a CUDA graph, both sides, us:
-// 16 rows 1024 x 512 q4_0 9.1 / 8.2, 1024 x 1024 9.5 / 11.7; 32 rows of q8_0 11.3 / 11.2, 12.3 / 16.9.  Up to 8 rows the mma.sync form holds out longer, except
-// where its weights are 8 bits wide (8 rows 1024 x 1024 9.4 / 12.7): 8 rows of q4_0 6144 x 4096 15.5 / 13.3, 8192 x 8192 23.1 / 26.1; fp16 4096 x 4096 16.1 / 13.3,
-// 6144 x 4096 18.7 / 19.3.  Rows of one or two K steps leave few CTAs and nothing to stream while the others meet: a step of 13 sequences at width 512,
-// whose only product this large is 3648 x 512, took 145 against 142 us, at width 1024 170 against 200.
-constexpr uint64_t BT_MIN_WEIGHTS = 1ull << 20, BT_MIN_WEIGHTS_FEW_ROWS = 1ull << 25, BT_MIN_WEIGHTS_SHORT = 1ull << 22;
+// Smallest products (weights) that go through tcgen05; below, launch and the meeting of CTAs cost more than gemv_batch.cu takes.  In a CUDA graph, mma.sync form / this
+// one, us: 9 rows 1664 x 640 q4_0 8.5 / 8.8, 1408 x 768 9.0 / 8.9, 1024 x 1024 11.0 / 9.0; q8_0 1664 x 640 11.0 / 8.8; fp16 10.3 / 10.3; 32 rows q4_0 13.7 / 12.1.
+// Up to 8 rows the mma.sync form holds out longer, except where its weights are 8 bits wide (8 rows q8_0 1664 x 640 10.0 / 8.7): 8 rows of q4_0 8256 x 4096 13.1 / 13.9,
+// 11712 x 4096 22.0 / 17.9; fp16 8256 x 4096 19.0 / 20.8, 16384 x 4096 35 / 29.
+// Below 640 columns it does, too: 9 rows q4_0 7360 x 288 7.1 / 7.7, 14592 x 288 7.7 / 7.8, 8192 x 512 9.2 / 7.7, but 7808 x 544 8.7 / 9.1, 10368 x 576 9.5 / 9.1;
+// fp16 8192 x 512 8.5 / 9.0, 16448 x 512 9.3 / 9.4, 7808 x 544 10.1 / 10.3; 32 rows q8_0 7360 x 288 9.8 / 10.7, 16384 x 256 10.2 / 8.6.
+constexpr uint64_t BT_MIN_WEIGHTS = 1ull << 20, BT_MIN_WEIGHTS_FEW_ROWS = 36ull << 20, BT_MIN_WEIGHTS_SHORT = 4ull << 20, BT_MIN_WEIGHTS_SHORT_FEW = 6ull << 20;
 constexpr uint32_t BT_SHORT_K = 640;
 
 namespace greta {

@@ -77,6 +77,26 @@ def test_products(g, name, M, N, K):
     assert np.array_equal(got[others], first[others])
 
 
+# Whole pairs of row tiles, one or two to a CTA; pairs in parts that do not divide their K steps; equal runs; few rows above the line of their own.
+@pytest.mark.parametrize("name", ["q4_0", "q8_0", "f16"])
+@pytest.mark.parametrize("M,N,K", [(9, 23400, 512), (12, 40001, 544), (32, 5900, 2080), (16, 1700, 8192), (10, 24000, 1312), (5, 5300, 7232)])
+def test_shares(g, name, M, N, K):
+    lib, rng = g.cuda(), np.random.default_rng(M + N + K)
+    w = _Weight(g, rng, name, N, K)
+    assert lib.greta_cuda_gemv_batch_route(w.fmt, M, N, K) == 1
+    x = rng.normal(0, 1, (M, K)).astype(np.float32)
+    xd, ws, y = g.DeviceBuffer.from_numpy(x), _ws(g, M, K), _out(g, M * N)
+    first = None
+    for _ in range(3):
+        g.check(lib.greta_cuda_gemv_batch(None, w.fmt, xd.ptr, None, 0.0, w.qs, w.d, None, y.ptr, M, N, K, 0, ws.ptr))
+        got = y.download(np.float32).reshape(M, N)
+        first = got.copy() if first is None else first
+        assert np.array_equal(got, first)
+    want = w.product(x)
+    for m in range(M):
+        assert max_abs_rel(got[m], want[m]) < TIGHT, m
+
+
 @pytest.mark.parametrize("name", ["q4_0", "q8_0"])
 @pytest.mark.parametrize("M,D,F", [(16, 1056, 1001), (32, 2080, 450), (8, 8192, 2100)])
 def test_gate_and_up(g, name, M, D, F):
