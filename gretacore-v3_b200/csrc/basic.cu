@@ -211,7 +211,9 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *logits, uint3
   pdl_wait();
   const uint32_t b = blockIdx.y, rank = blockIdx.x, ctas = gridDim.x;  // sequence: its own logits row, result, position, counter and output list
   logits += (size_t)b * n;
-  if (code && b == 0 && rank == 0 && threadIdx.x == 0) out[gridDim.y] = __ldcg(code);
+  const bool tells = code && b == 0 && rank == 0 && threadIdx.x == 0;
+  int told = 0;
+  if (tells) told = __ldcg(code);  // stored at the end: nothing waits for it
   out += b;
   if (d_pos) d_pos += b;
   if (d_count) d_count += b;
@@ -270,6 +272,7 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float *logits, uint3
     }
     if (l == 0) {
       *out = (int32_t)bi;
+      if (tells) out[gridDim.y] = told;
       if (d_count) {
         uint32_t c = *d_count;
         if (out_tokens && c < out_capacity) out_tokens[c] = (int32_t)bi;
