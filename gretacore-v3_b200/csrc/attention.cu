@@ -56,14 +56,16 @@ __global__ void __launch_bounds__(CL_WARPS * 32) attn_cluster_kernel(const AttnP
   cg::cluster_group cluster = cg::this_cluster();
   pdl_launch_dependents();
   const uint32_t split = cluster.block_rank(), head = blockIdx.y, qi = blockIdx.z;
-  // This CTA's rows start their way from HBM to L2 while it still waits.  Only hints: neither the position nor the rows need be final yet.  Not over
-  // small caches, where it gains nothing (279 positions 486 -> 489 us for 8 steps; 520 positions 2021 -> 2000).
-  if (sizeof(KV) == 2 && p.max_seq >= 512 && head % (p.H / p.Hkv) == 0) {
+  // This CTA's first rows start their way from HBM to L2 while it still waits; the rest would come in front of the rows that are needed first.  Only hints:
+  // neither the position nor the rows need be final yet.  One decoder layer of 32 heads of 128, us without / 32 KB of keys and of values / all rows: 128 keys 43.5 /
+  // 43.1 / 43.1, 2048 keys 51.4 / 50.6 / 50.8, 4096 keys 58.6 / 57.8 / 61.5; 8 KV heads, 4096 keys 54.1 / 53.9 / 54.7; width 512, 512 keys 15.6 / 15.6 / 15.6.
+  constexpr uint32_t AHEAD = 32768;
+  if (sizeof(KV) == 2 && head % (p.H / p.Hkv) == 0) {
     const uint32_t L = min((p.d_pos ? __ldcg(p.d_pos + qi * p.pos_stride) : p.len0) + qi * p.len_step, p.max_seq), chunk = (L + CL_SPLITS - 1) / CL_SPLITS;
     const uint32_t k0 = min(L, split * chunk), k1 = min(L, k0 + chunk);
     const size_t at = ((size_t)qi * p.seq_stride + ((size_t)(head / (p.H / p.Hkv)) * p.max_seq + k0) * Dh) * 2;
     const char *kp = reinterpret_cast<const char *>(p.kc) + at, *vp = reinterpret_cast<const char *>(p.vc) + at;
-    for (uint32_t b = threadIdx.x * 128; b < (k1 - k0) * Dh * 2; b += CL_WARPS * 32 * 128) {
+    for (uint32_t b = threadIdx.x * 128; b < min((k1 - k0) * Dh * 2, AHEAD); b += CL_WARPS * 32 * 128) {
       asm volatile("prefetch.global.L2 [%0];" ::"l"(kp + b));
       asm volatile("prefetch.global.L2 [%0];" ::"l"(vp + b));
     }
@@ -524,7 +526,8 @@ static int attn_prefill_impl(greta_stream_t stream, const float *q, const void *
   p.H = H; p.Hkv = Hkv; p.max_seq = max_seq; p.scale = scale; p.splits = 1; p.len_step = 1;
   // Prompts run on the tensor cores; a few positions, or the switch off, take one CTA per (position, head) on the decode inner loop.
   if (tuning().attn_mma && S >= 8 && (Dh == 64 || Dh == 128) && aligned16(q) && aligned16(kc) && aligned16(vc) && aligned16(o)) {
-    // tcgen05 above 512 keys: 1531 rows of 32 heads 98 against 256 us, 2048 rows of 64 heads of 64 168 against 365.  It would pay from 128 keys on (a
+    // tcgen05 above 512 keys: 1531 rows of 32 heads 98 against 256 us, 2048 rows of 64 heads of 64 168 against 365; few rows behind a long cache, 32 heads
+    // of 128 over 8: 8 rows behind 600 / 1000 / 4000 keys 14 / 18 / 53 against 42 / 67 / 253, 64 rows 20 / 24 / 58 against 47 / 74 / 262.  It would pay from 128 keys on (a
     // 512-token prompt of four 7B layers 1104 against 1190 us).  The line lies higher because the ids of the 512-token 7B run hang on a top-2
     // gap of 4.4e-6, less than what the products' sums leave open: with the smaller rounding error of this form one id of 128 is another.
     if (greta_cuda_attn_prefill_route(S, pos0, Dh) && (!o16 || aligned16(o16)))
