@@ -32,7 +32,9 @@ constexpr uint32_t MIN_TOKENS = 80;
 // waiting for it (scan j - 2, which read its half, has ended: scan j - 1 waited for prepare j - 1, and that for scan j - 2), and only its first CTA
 // waits for scan j - 1, at its end, so that the end of prepare j implies that of scan j - 1.  What other kernels of this chain may have
 // read before is loaded past L1.
-// 2048 tokens of 32 heads 64 x 64: 154 us with 768 tokens, 159 with 512, 178 with 1024, 205 with 256; 1337 of 16 heads 128 x 128: 106, 116, 115, 130.
+// 2048 tokens, us with 256 / 512 / 768 / 1024 tokens (in a graph, inputs in L2): general form, heads of 64: 8 heads 90 / 84 / 85 / 84, 32 heads 193 / 151 / 144 / 143, 64 heads
+// 307 / 281 / 290 / 282; heads of 128: 8 heads 139 / 134 / 142 / 147, 16 heads 229 / 214 / 215 / 214, 64 heads 849 / 892 / 873 / 878; gated, heads of 128: 8 heads
+// 118 / 116 / 118 / 118, 16 heads 185 / 162 / 153 / 146, 64 heads 629 / 574 / 560 / 554.  Between 512 and 1024 there is little to choose.
 constexpr uint32_t SLICE = 768;
 
 __host__ __device__ constexpr uint32_t pad16(uint32_t v) { return (v + 15u) & ~15u; }

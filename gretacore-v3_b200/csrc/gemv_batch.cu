@@ -1,7 +1,7 @@
 // Batched decode matmul: y[M x N] = x[M x K] * dequant(W)^T for M = 2..32 activation rows (one per
 // sequence of a decode batch), with the same RMSNorm prologue and RoPE / KV-cache / SwiGLU / residual
-// epilogues as the single-row GEMV.  The weights are streamed from HBM ONCE for all M rows, so the work
-// stays HBM-bound (0.5625 B per weight for Q4_0) where a per-row GEMV would read them M times.
+// epilogues as the single-row GEMV.  The weights are streamed from HBM ONCE for all M rows, where a per-row GEMV
+// would read them M times (0.5625 B per weight for Q4_0).
 //
 //   * A CTA owns 128 or 256 weight rows (16-row tiles, one or two per warp, 8 warps) over one slice of K.
 //     Weight tiles travel global -> shared with 16-byte cp.async copies into a per-warp ring of 8-block
@@ -10,10 +10,13 @@
 //   * One weight block meets all M activation rows in the tensor cores: the nibbles (bytes, halves) are
 //     unpacked to the exact small integers q - 8 as fp16 and fed to mma.sync m16n8k16 as the 16-row
 //     operand, the activations are the 8-column operand, fp32 accumulation over the 32 values of the
-//     block; the block's fp16 scale is applied to the 16 x 8 block sums with fp32 FMAs.  Per-block
-//     scales rule out accumulating across blocks inside the tensor core (and with it TMEM): the block
-//     sums have to come back to registers every 32 values, which is what mma.sync does by construction.
-//     The kernel is bound by HBM and by instruction issue, not by the tensor pipe.
+//     block; the block's fp16 scale is applied to the 16 x 8 block sums with fp32 FMAs.  The block
+//     sums have to come back to fp32 registers every 32 values, which mma.sync does by construction and
+//     which caps this kernel at that instruction's rate (0.2 of the memory bandwidth for 16 rows of Q4_0).
+//   * With a workspace and k_slices 0, large products go to gemv_tc.cu instead, which reads the block sums out
+//     of tensor memory.  What stays here: small products (below a million weights, 37 million up to 8 rows of
+//     4-bit or fp16 weights; the lines and both sides' times stand in gemv_tc.cuh), forced k_slices, and calls
+//     without a workspace.
 //   * Activations keep fp32 precision: each value is split into two fp16 numbers, hi = half(x * s) and
 //     lo = half(x * s - hi), s a power of two chosen per row and per K-chunk so that the chunk's largest
 //     value sits near 2^14; both parts run through the same accumulator.  Every product is exact; the

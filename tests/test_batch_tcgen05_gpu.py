@@ -1,6 +1,8 @@
 """Batched products that go through tcgen05 (a million weights or more, with workspace): row tiles and K steps that are not whole, both widths of the
 activation operand (16 and 32 rows), row tiles shared by many CTAs and shares that end inside a pair of tiles, every epilogue and weight format.
 Bars as in test_batch_gpu.py: 2e-5 (observed about 3e-7), exact integer weights and activations of at least 22 bits, summed in fp32."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -141,6 +143,38 @@ def test_queries_keys_and_values(g, name, M, H, Hkv, Dh, D):
                                                            None, None, None, M, H, Hkv, Dh, max_seq, 10000.0, D, ws.ptr))
     for buf, w in ((q_out, wq), (k_out, wk), (v_out, wv)):
         assert max_abs_rel(buf.download(np.float32).reshape(M, -1), w.product(x)) < TIGHT
+
+
+def test_products_on_two_streams(g):
+    """Each stream with a workspace of its own, captured into a graph on the second: the results of the default stream."""
+    lib, rng, M, N, K = g.cuda(), np.random.default_rng(8), 16, 6000, 2080
+    w = _Weight(g, rng, "q4_0", N, K)
+    assert lib.greta_cuda_gemv_batch_route(w.fmt, M, N, K) == 1
+    xd = g.DeviceBuffer.from_numpy(rng.normal(0, 1, (M, K)).astype(np.float32))
+    call = lambda stream, ws, y: g.check(lib.greta_cuda_gemv_batch(stream, w.fmt, xd.ptr, None, 0.0, w.qs, w.d, None, y.ptr, M, N, K, 0, ws.ptr))
+    ws, y = _ws(g, M, K), _out(g, M * N)
+    call(None, ws, y)
+    want = y.download(np.float32)
+    streams, spaces, outs = [C.c_void_p(), C.c_void_p()], [_ws(g, M, K) for _ in range(2)], [_out(g, M * N) for _ in range(2)]
+    graph, ready = C.c_void_p(), C.c_void_p()
+    for s in streams:
+        g.check(lib.greta_cuda_stream_create(C.byref(s)))
+    g.check(lib.greta_cuda_device_synchronize())
+    g.check(lib.greta_cuda_graph_capture_begin(streams[1]))
+    call(streams[1], spaces[1], outs[1])
+    g.check(lib.greta_cuda_graph_capture_end(streams[1], C.byref(graph)))
+    g.check(lib.greta_cuda_graph_instantiate(graph, C.byref(ready)))
+    for _ in range(8):
+        call(streams[0], spaces[0], outs[0])
+        g.check(lib.greta_cuda_graph_launch(ready, streams[1]))
+    for s in streams:
+        g.check(lib.greta_cuda_stream_synchronize(s))
+    for o in outs:
+        assert np.array_equal(o.download(np.float32), want)
+    g.check(lib.greta_cuda_graph_exec_destroy(ready))
+    g.check(lib.greta_cuda_graph_destroy(graph))
+    for s in streams:
+        g.check(lib.greta_cuda_stream_destroy(s))
 
 
 def test_a_batch_reports_a_product_that_gave_up(g):
