@@ -441,11 +441,9 @@ bool BlockScheduler::allocate_hybrid_activations(std::string *err) {
   // Scratch of the chunked scans (120 MB for 32 heads of 64): last, and only where as much again stays free for what is loaded afterwards.  Without it
   // prompts take the scans token by token.
   w.scan_scratch.free();
-  Buffer room;
-  if (scan && room.allocate(2 * scan, BufferUsage::DeviceOnly, GretaDataType::FP32, nullptr)) {
-    room.free();
+  size_t free_bytes = 0, total_bytes = 0;
+  if (scan && greta_cuda_mem_info(&free_bytes, &total_bytes) == GRETA_OK && free_bytes / 2 >= scan)
     w.scan_scratch.allocate(scan, BufferUsage::DeviceOnly, GretaDataType::FP32, nullptr);
-  }
   GRETA_TRY(greta_cuda_device_synchronize(), "allocate_activations");
   invalidate_graph();
   return true;

@@ -191,6 +191,11 @@ int greta_cuda_free(void *ptr) {
   if (ptr) GRETA_CUDA_TRY(cudaFree(ptr));
   return GRETA_OK;
 }
+int greta_cuda_mem_info(size_t *free_bytes, size_t *total_bytes) {
+  GRETA_REQUIRE(free_bytes && total_bytes, "mem_info: null out pointer");
+  GRETA_CUDA_TRY(cudaMemGetInfo(free_bytes, total_bytes));
+  return GRETA_OK;
+}
 int greta_cuda_malloc_host(void **ptr, size_t bytes) {
   GRETA_REQUIRE(ptr, "malloc_host: null out pointer");
   *ptr = nullptr;

@@ -87,6 +87,8 @@ GRETA_API int greta_cuda_memcpy_2d_d2d(void *dst, size_t dst_pitch, const void *
 /* height rows of width bytes from a pitched device array to a pitched host array; blocks. */
 GRETA_API int greta_cuda_memcpy_2d_d2h_sync(void *dst, size_t dst_pitch, const void *src, size_t src_pitch, size_t width, size_t height);
 GRETA_API int greta_cuda_memcpy_h2d_sync(void *dst, const void *src, size_t bytes);
+/* Bytes of the current device's memory that are free, and all of it. */
+GRETA_API int greta_cuda_mem_info(size_t *free_bytes, size_t *total_bytes);
 GRETA_API int greta_cuda_memcpy_d2h_sync(void *dst, const void *src, size_t bytes);
 GRETA_API int greta_cuda_memset(void *dst, int value, size_t bytes, greta_stream_t stream);
 GRETA_API int greta_cuda_stream_create(greta_stream_t *stream);

@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 def _free():
     free, total = C.c_size_t(), C.c_size_t()
-    assert C.CDLL("libcuda.so.1").cuMemGetInfo_v2(C.byref(free), C.byref(total)) == 0
+    lib = load_package().ffi.cuda()
+    assert lib.greta_cuda_mem_info(C.byref(free), C.byref(total)) == 0 and free.value <= total.value
     return free.value
 
 
