@@ -89,6 +89,7 @@ GRETA_API int greta_model_forward_logits(greta_model_t m, const int32_t *tokens,
                                          uint32_t n_rows, float *out);
 /* forward() of a prompt of n tokens from position 0, `reps` times between two events; *ms = device time of one. */
 GRETA_API int greta_model_forward_timed(greta_model_t m, const int32_t *tokens, uint32_t n, uint32_t reps, float *ms);
+/* The next three fail, once, where a bounded wait of the steps before them gave up (BlockScheduler::finish). */
 GRETA_API int greta_model_get_logits(greta_model_t m, float *out, uint32_t n);           /* get_logits() -> host */
 GRETA_API int greta_model_get_hidden(greta_model_t m, float *out, uint32_t row, uint32_t n); /* get_hidden_state() row -> host */
 GRETA_API int greta_model_sample_greedy(greta_model_t m, int32_t *id);                   /* sample_greedy_gpu */
